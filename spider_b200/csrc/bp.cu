@@ -27,8 +27,7 @@ namespace spi {
 struct SliceDesc {
   float dm[6];  // DMS(1:6): first two columns of the (symmetrised) rotation
   int img;      // image index inside the chunk
-  short grid;   // target grid (BP 32F half set)
-  short cols;   // insertion order of the x4 kernels: 0 row by row, 1 column by column
+  int grid;     // target grid (BP 32F half set)
 };
 static_assert(sizeof(SliceDesc) == 32, "slice descriptor is 32 bytes");
 
@@ -1070,35 +1069,10 @@ __global__ void __launch_bounds__(512) insert_xlane_kernel(const void* __restric
 }
 
 // ----------------------------------------------------------------------------
-// Insert, four lanes per pixel over the nonzero taps.  The generalised
-// Kaiser-Bessel table is zero from distance ~1.8 on (0.9 of the two-voxel
-// half width), so along each axis the tap at offset -2 is nonzero only when
-// the coordinate lies more than 0.2 below its nearest voxel and the tap at +2
-// only when it lies more than 0.2 above: at most four of the five taps are
-// nonzero, in the window [-2, 1] or [-1, 2].  A warp takes one row J of one
-// slice, eight pixels at a time; lanes 4g..4g+3 share pixel I0+g, lane 4g+q
-// owns x tap XS+q of the window, and each lane loops over the 4 x 4 (Y, Z)
-// window.  Window starts are read from the same table lookups the taps use
-// (offset -2 nonzero => window [-2, 1]); the host verifies that the table is
-// zero beyond distance 2, which makes the window exact.  Compared with five
-// lanes over all 5 x 5 (Y, Z) taps this issues 2 instead of 4.2 atomic
-// instructions per pixel and uses every lane.  Each voxel and weight (and
-// the reflected points of oneline.f:118-150) is computed as in insert_kernel;
-// taps outside the window have zero weight, which the reference skips too.
-__device__ __forceinline__ float kb_tap(const float* tab, float v, int k, float fltb) {
-  return tab[nint_pos(__fmul_rn(fabsf(__fsub_rn(v, (float)k)), fltb))];
-}
-// The same lookup in a table cut after entry `last`, which (like every entry
-// after it) is zero: for a table kb_window4_ok accepts, the result is the
-// same as kb_tap's.
-__device__ __forceinline__ float kb_tap_cut(const float* tab, float v, int k, float fltb, int last) {
-  return tab[min(nint_pos(__fmul_rn(fabsf(__fsub_rn(v, (float)k)), fltb)), last)];
-}
-
 // G[i] += v as one 16-byte reduction in L2 (red.global.add.v4.f32).  The
-// address is converted to the global window explicitly: the multi-class
-// kernel takes its grid pointers from shared memory, and on such a generic
-// pointer atomicAdd(float4*) was not compiled to the vector reduction
+// address is converted to the global window explicitly: insert_x4_kernel
+// takes its grid pointer from shared memory, and on such a generic pointer
+// atomicAdd(float4*) was not compiled to the vector reduction
 // (measured: 1.9x the instructions and no L2 reduction requests; 205
 // against 156 ms for the same 10,000 images at 256^3).
 __device__ __forceinline__ void red_add_v4(float4* p, float4 v) {
@@ -1106,205 +1080,16 @@ __device__ __forceinline__ void red_add_v4(float4* p, float4 v) {
                "f"(v.y), "f"(v.z), "f"(v.w));
 }
 
-// The largest m >= 0 with m * m < rem (rem > 0).
-__device__ __forceinline__ int isqrt_below(int rem) {
-  // approximate square root (no IEEE slow path); the two loops make m exact
-  float f;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"((float)(rem - 1)));
-  int m = (int)f;
-  while (m > 0 && m * m >= rem) --m;
-  while ((m + 1) * (m + 1) < rem) ++m;
-  return m;
-}
+}  // namespace spi
+#include "slab.cuh"   // insert_x4_kernel
+namespace spi {
 
-// One line of one slice, eight pixels at a time, as described above: the
-// body of insert_x4_kernel and insert_mc_kernel.  Line r (0 <= r < N) is row
-// J = r - NX + 1 (pixels consecutive in I), or, for a slice whose
-// descriptor says cols, half of column I = r / 2 (pixels consecutive in J:
-// J >= 0 for even r, J < 0 for odd r).  The eight pixels of a step then lie
-// along the slice's second axis (DMS(4:6)) instead of its first (DMS(1:3)).
-// The host picks, per slice, the axis whose z component is smaller: a step
-// along z puts the eight pixels' atomics in eight grid planes 2 MB apart
-// (measured at 256^3: rows along z 45.5k images/s, along x or y 65k).  Each
-// pixel's taps and weights are the same in both orders.
-template <bool BF16, int CUT = 0>
-__device__ __forceinline__ void insert_line_x4(const void* __restrict__ spec, const SliceDesc& sd,
-                                               float4* __restrict__ G, int r, int nx, const float* tab, float fltb,
-                                               int g, int q, int gl) {
-  // CUT > 0: the table holds entries 0..CUT-1 only (see kb_tap_cut)
-  auto tap = [&](float v, int k) { return CUT ? kb_tap_cut(tab, v, k, fltb, CUT - 1) : kb_tap(tab, v, k, fltb); };
-  const int N = 2 * nx, N2 = nx, LN2 = 2;
-  const int NN4 = N * N / 4;
-  const float fN = (float)N;
-  const size_t rowlen = (size_t)(nx + 1);
-  const size_t plane = (size_t)N * rowlen;
-  const size_t spec0 = (size_t)sd.img * plane;
-  // pixel k of the line: (I, J) = (i0 + di * k, j0 + dj * k), k < cnt; the
-  // pixels inside the half disc of oneline.f's loops (I >= 0, I*I + J*J <
-  // NN4, no I = 0 with J < 0)
-  int i0, j0, di, dj, cnt;
-  if (!sd.cols) {
-    j0 = r - nx + 1; i0 = 0; di = 1; dj = 0;                 // J = -NX+1 .. NX
-    cnt = (j0 * j0 < NN4) ? isqrt_below(NN4 - j0 * j0) + 1 : 0;
-  } else {
-    i0 = r >> 1; di = 0;                                      // I = 0 .. NX-1
-    const int jm = isqrt_below(NN4 - i0 * i0);
-    if (r & 1) { j0 = -1; dj = -1; cnt = i0 == 0 ? 0 : jm; }
-    else { j0 = 0; dj = 1; cnt = jm + 1; }
-  }
-#pragma unroll 1
-  for (int k0 = 0; k0 < cnt; k0 += 8) {   // warp-uniform
-    const int k = k0 + g;
-    const int I = i0 + di * k, J = j0 + dj * k;
-    bool ok = k < cnt && !(I == 0 && J < 0);
-    const float fI = (float)I, fJ = (float)J;
-    float xnew = __fadd_rn(__fmul_rn(fI, sd.dm[0]), __fmul_rn(fJ, sd.dm[3]));
-    float ynew = __fadd_rn(__fmul_rn(fI, sd.dm[1]), __fmul_rn(fJ, sd.dm[4]));
-    float znew = __fadd_rn(__fmul_rn(fI, sd.dm[2]), __fmul_rn(fJ, sd.dm[5]));
-    float br = 0.0f, bi = 0.0f;
-    if (ok) {
-      const int JP = (J >= 0) ? J : N + J;
-      const float2 sp = load_spec<BF16>(spec, spec0 + (size_t)JP * rowlen + I);
-      br = sp.x;
-      bi = -sp.y;   // SPIDER forward sign = conjugate of the cuFFT R2C output
-    }
-    if (xnew < 0.0f) {
-      xnew = -xnew; ynew = -ynew; znew = -znew;
-      bi = -bi;
-    }
-    const int ixn = __float2int_rz(__fadd_rn(__fadd_rn(xnew, 0.5f), fN)) - N;
-    const int iyn = __float2int_rz(__fadd_rn(__fadd_rn(ynew, 0.5f), fN)) - N;
-    const int izn = __float2int_rz(__fadd_rn(__fadd_rn(znew, 0.5f), fN)) - N;
-    ok = ok && ixn <= (N2 - LN2 - 1) && iyn >= (-N2 + 2 + LN2) && iyn <= (N2 - LN2 - 1) &&
-         izn >= (-N2 + 2 + LN2) && izn <= (N2 - LN2 - 1);
-    if (!ok) { xnew = ynew = znew = 0.0f; }   // keeps the lookups below in range; no taps follow
-    const int ix0 = ok ? ixn : 0, iy0 = ok ? iyn : 0, iz0 = ok ? izn : 0;
-    const int xs = tap(xnew, ix0 - 2) != 0.0f ? ix0 - 2 : ix0 - 1;
-    const int ys = tap(ynew, iy0 - 2) != 0.0f ? iy0 - 2 : iy0 - 1;
-    const int zs = tap(znew, iz0 - 2) != 0.0f ? iz0 - 2 : iz0 - 1;
-    const float tx = tap(xnew, xs + q);
-    const float tyq = tap(ynew, ys + q);
-    const float tzq = tap(znew, zs + q);
-    float ty[4], tz[4];
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      ty[l] = __shfl_sync(0xffffffffu, tyq, gl + l);
-      tz[l] = __shfl_sync(0xffffffffu, tzq, gl + l);
-    }
-    if (!ok || tx == 0.0f) continue;
-    // main tap at (ixp, iyp, izp), or for ixp < 0 the reflected point
-    // (-ixp, -iyp, -izp) with the conjugate value
-    const int ixp = xs + q;
-    const bool refl = ixp < 0;
-    const float bis = refl ? -bi : bi;
-    const int ixa = refl ? -ixp : ixp;
-#pragma unroll
-    for (int lz = 0; lz < 4; ++lz) {
-      if (tz[lz] == 0.0f) continue;
-      const int izp = zs + lz;
-      const int iza = refl ? ((izp > 0) ? N - izp : -izp) : ((izp >= 0) ? izp : N + izp);
-#pragma unroll
-      for (int ly = 0; ly < 4; ++ly) {
-        const float tyz = __fmul_rn(ty[ly], tz[lz]);
-        if (tyz == 0.0f) continue;
-        const int iyp = ys + ly;
-        const int iya = refl ? ((iyp > 0) ? N - iyp : -iyp) : ((iyp >= 0) ? iyp : N + iyp);
-        const float wg = __fmul_rn(tx, tyz);
-        if (wg != 0.0f)
-          red_add_v4(G + ((size_t)iza * N + iya) * rowlen + ixa,
-                     make_float4(__fmul_rn(br, wg), __fmul_rn(bis, wg), wg, 0.0f));
-      }
-    }
-  }
-}
-
-// 48 registers: 0.6% faster at 256^3 than the compiler's own choice of 64
-// (measured), with no spills; launches use at most 512 threads.
-template <bool BF16>
-__global__ void __maxnreg__(48) insert_x4_kernel(const void* __restrict__ spec, const SliceDesc* __restrict__ slices,
-                                                 int nslices, int nx, const float* __restrict__ kbtab, float fltb,
-                                                 float4* __restrict__ g0, float4* __restrict__ g1,
-                                                 unsigned long long* __restrict__ work) {
-  extern __shared__ float tab[];
-  for (int i = threadIdx.x; i < 5000; i += blockDim.x) tab[i] = kbtab[i];
-  __syncthreads();
-
-  const int N = 2 * nx;
-  const int lane = threadIdx.x & 31;
-  const int g = lane >> 2;          // pixel of the group of eight
-  const int q = lane & 3;           // x tap of the window
-  const int gl = lane & ~3;         // first lane of the group
-  const long long nitems = (long long)nslices * N;
-
-  for (;;) {
-    unsigned long long it = 0;
-    if (lane == 0) it = atomicAdd(work, 1ull);
-    const long long item = (long long)__shfl_sync(0xffffffffu, it, 0);
-    if (item >= nitems) break;
-    const int s = (int)(item / N);
-    const SliceDesc sd = slices[s];
-    insert_line_x4<BF16>(spec, sd, sd.grid ? g1 : g0, (int)(item % N), nx, tab, fltb, g, q, gl);
-  }
-}
-
-// ----------------------------------------------------------------------------
-// Insert for several classes of different box sizes in one launch (BP 32F of
-// each class, the image loop bp32f.f:802-913 run for all classes together).
-// The work items are the rows of every class's slices, class after class;
-// a row finds its class by its item index and takes that class's box size,
-// table (one shared-memory copy per distinct box size), spectra and grids.
-// Each row is inserted exactly as insert_x4_kernel inserts it.
-struct McClass {
-  const void* spec;            // spectra of the class's images in this launch
-  const SliceDesc* slices;     // the class's slice descriptors
-  float4* g0;                  // grids the taps go to (half-set 1 and 2)
-  float4* g1;
-  long long item0;             // first work item (row) of the class
-  int nx, nslices, tab, pad;   // box size, slices, table index
-};
-static_assert(sizeof(McClass) == 56, "class descriptor is 56 bytes");
-constexpr int kMcMaxClass = 16, kMcMaxTab = 8;
-// Entries of a table the multi-class kernel keeps: a table kb_window4_ok
-// accepts is zero from floor(2 * FLTB) - 1 = 3331 on (FLTB = 4999/3), so
-// 3,332 entries (13 KB) hold every nonzero value and a zero to clamp to;
-// eight tables then fit two CTAs per SM.
-constexpr int kMcTab = 3332;
-
-template <bool BF16>
-__global__ void __launch_bounds__(512) insert_mc_kernel(const McClass* __restrict__ cls, int ncls, long long nitems,
-                                                        const float* __restrict__ tabs, const float* __restrict__ fltbs,
-                                                        int ntab, unsigned long long* __restrict__ work) {
-  extern __shared__ float tab[];   // [ntab][kMcTab]
-  __shared__ McClass sc[kMcMaxClass];
-  __shared__ float sfl[kMcMaxTab];
-  for (int i = threadIdx.x; i < kMcTab * ntab; i += blockDim.x) tab[i] = tabs[(i / kMcTab) * 5000 + i % kMcTab];
-  if (threadIdx.x < ncls) sc[threadIdx.x] = cls[threadIdx.x];
-  if (threadIdx.x < ntab) sfl[threadIdx.x] = fltbs[threadIdx.x];
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int g = lane >> 2, q = lane & 3, gl = lane & ~3;
-  for (;;) {
-    unsigned long long it = 0;
-    if (lane == 0) it = atomicAdd(work, 1ull);
-    const long long item = (long long)__shfl_sync(0xffffffffu, it, 0);
-    if (item >= nitems) break;
-    int c = 0;
-    while (c + 1 < ncls && sc[c + 1].item0 <= item) ++c;
-    const McClass& C = sc[c];
-    const int N = 2 * C.nx;
-    const long long local = item - C.item0;
-    const SliceDesc sd = C.slices[local / N];
-    insert_line_x4<BF16, kMcTab>(C.spec, sd, sd.grid ? C.g1 : C.g0, (int)(local % N), C.nx, tab + kMcTab * C.tab,
-                                 sfl[C.tab], g, q, gl);
-  }
-}
-
-// True when the table is zero for every distance >= 2 (index nint(2*fltb)
-// and above, less one for rounding), the condition under which at most four
-// consecutive taps of the five are nonzero (insert_x4_kernel).
+// True when the table is zero from distance 1.805 on, as FILLBESSIL's are
+// (0.9 of the two-voxel half width): at most four consecutive taps of the five
+// are then nonzero and columns within kSlabR of a pixel hold them all
+// (insert_x4_kernel).
 static bool kb_window4_ok(const KBTab& kb) {
-  const int i0 = std::max(0, (int)std::floor(2.0 * kb.fltb) - 1);
-  for (int i = i0; i < 5000; ++i)
+  for (int i = std::max(0, (int)std::floor(1.805 * kb.fltb)); i < 5000; ++i)
     if (kb.tab[i] != 0.0f) return false;
   return true;
 }
@@ -1879,7 +1664,6 @@ void bp_release(spi_ctx* c) {
   c->spec_tmp.release();
   c->slices.release();
   c->workctr.release();
-  c->mc_params.release();
   c->mc_host.release();
   c->cplx.release();
   c->real3.release();
@@ -2167,18 +1951,20 @@ int spi_bp_open(spi_ctx* c, int nx, int ngrids, const float* sym_angles, int nsy
                    : strcmp(m, "xlane") == 0 ? 2 : strcmp(m, "tilefx") == 0 ? 4 : def_mode;
     const char* o = getenv("SPI_SLICE_ORDER");
     c->slice_order = (o && strcmp(o, "input") == 0) ? 0 : 1;
-    const char* lo = getenv("SPI_INSERT_ORDER");
-    c->line_order = !lo ? 1 : strcmp(lo, "rows") == 0 ? 0 : strcmp(lo, "cols") == 0 ? 2 : 1;
     const char* mp = getenv("SPI_INSERT_MAP");
     c->insert_seg_map = (mp && strcmp(mp, "seg") == 0) ? 1 : 0;
-    // The insertion is limited by L2 atomics, not by occupancy.  Measured on
-    // 4,096 images: the x-lane kernel is best at 24 warps/SM for 128^3 and 16
+    // The per-tap kernels are limited by L2 atomics, not by occupancy.  Measured
+    // on 4,096 images: the x-lane kernel is best at 24 warps/SM for 128^3 and 16
     // for 64^3 and 256^3; the direct kernel at 24 warps/SM for 64^3, 8 for
-    // 128^3-192^3 and 4 for 256^3.
+    // 128^3-192^3 and 4 for 256^3.  The column kernel runs as many CTAs as fit.
     int def_threads = 256, def_bps = (nx > 96 && nx <= 160) ? 3 : 2;
     if (c->insert_mode == 1) {
       def_threads = nx <= 96 ? 256 : 128;
       def_bps = nx <= 96 ? 3 : nx <= 224 ? 2 : 1;
+    }
+    if (c->insert_mode == 3) {
+      def_threads = kSlabThreads;
+      def_bps = kSlabBlocks;
     }
     c->insert_threads = env_int("SPI_INSERT_THREADS", def_threads);
     if (c->insert_threads != 64 && c->insert_threads != 128 && c->insert_threads != 256 && c->insert_threads != 512)
@@ -2381,6 +2167,56 @@ static int insert_blocks(spi_ctx* c, K kernel, int threads, size_t smem, int cap
   return c->sm_count * std::max(per_sm, 1);
 }
 
+// One class of a column insertion: the slices of one reconstruction
+static SlabClass slab_class(const spi_ctx* c, const void* spec, const SliceDesc* sl, int nslices, float4* g0, float4* g1) {
+  SlabClass m{};
+  m.spec = spec;
+  m.slices = sl;
+  m.g0 = g0;
+  m.g1 = g1;
+  m.tab = c->kbtab.as<float>();
+  m.nx = c->nx;
+  m.nslices = nslices;
+  m.fltb = c->kb.fltb;
+  return m;
+}
+
+// Work items of the classes: a slice's row of tiles each, or its parts when
+// all rows together would give the launch's CTAs fewer than eight items (the
+// tail of a launch is about half an item per CTA: 200 slices at 64^3 0.148
+// against 0.176 ms with whole rows).  Returns their number.
+static long long slab_items(int sm_count, SlabClass* cls, int ncls) {
+  auto rows_of = [](const SlabClass& m) { return (long long)m.nslices * ((2 * m.nx + kSlabTile - 1) / kSlabTile); };
+  long long rows = 0, items = 0;
+  for (int k = 0; k < ncls; ++k) rows += rows_of(cls[k]);
+  const long long want = 8LL * kSlabBlocks * sm_count;
+  for (int k = 0; k < ncls; ++k) {
+    const long long most = (cls[k].nx + kSlabTile - 1) / kSlabTile;
+    cls[k].parts = (int)std::max(1LL, std::min(most, rows > 0 ? (want + rows - 1) / rows : 1LL));
+    cls[k].item0 = items;
+    items += rows_of(cls[k]) * cls[k].parts;
+  }
+  return items;
+}
+
+// insert_x4_kernel over the items of a, persistent; `work` is zeroed first
+static int launch_slab(spi_ctx* c, const SlabArgs& a, bool bf16, unsigned long long* work, int per_sm, cudaStream_t st) {
+  SPI_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), st));
+  auto go = [&](auto kern, size_t smem) -> int {
+    // the attribute is per device and kernel; set once (several threads may race here harmlessly)
+    static std::atomic<unsigned long long> attr_done[2];
+    const unsigned long long bit = 1ull << (c->device & 63);
+    if (!(attr_done[bf16].load() & bit)) {
+      SPI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      attr_done[bf16].fetch_or(bit);
+    }
+    kern<<<insert_blocks(c, kern, kSlabThreads + 32, smem, per_sm), kSlabThreads + 32, smem, st>>>(a, work);
+    return check_kernel("insert_x4_kernel");
+  };
+  if (bf16) return go(insert_x4_kernel<true>, sizeof(SlabSmem<true>));
+  return go(insert_x4_kernel<false>, sizeof(SlabSmem<false>));
+}
+
 static int launch_insert(spi_ctx* c, const SliceDesc* sl, int nslices, float4* g1) {
   const void* spec = c->spectra.p;
   const int nx = c->nx;
@@ -2400,15 +2236,12 @@ static int launch_insert(spi_ctx* c, const SliceDesc* sl, int nslices, float4* g
                                threads, smem, c->stream>>>(spec, sl, nslices, nx, tab, fltb, g0, g1,
                                                            c->insert_seg_map);
     } else if (c->insert_mode == 3) {
+      SlabArgs a{};
+      a.ncls = 1;
+      a.cls[0] = slab_class(c, spec, sl, nslices, g0, g1);
+      a.nitems = slab_items(c->sm_count, a.cls, 1);
       SPI_TRY(c->workctr.ensure(sizeof(unsigned long long)));
-      auto* work = c->workctr.as<unsigned long long>();
-      SPI_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), c->stream));
-      if (c->bf16)
-        insert_x4_kernel<true><<<insert_blocks(c, insert_x4_kernel<true>, threads, smem, c->insert_blocks_per_sm),
-                                 threads, smem, c->stream>>>(spec, sl, nslices, nx, tab, fltb, g0, g1, work);
-      else
-        insert_x4_kernel<false><<<insert_blocks(c, insert_x4_kernel<false>, threads, smem, c->insert_blocks_per_sm),
-                                  threads, smem, c->stream>>>(spec, sl, nslices, nx, tab, fltb, g0, g1, work);
+      SPI_TRY(launch_slab(c, a, c->bf16, c->workctr.as<unsigned long long>(), c->insert_blocks_per_sm, c->stream));
     } else {
       // row counter of this launch (launches on the library stream are serialised)
       SPI_TRY(c->workctr.ensure(sizeof(unsigned long long)));
@@ -2471,18 +2304,6 @@ static int ensure_pipeline_events(spi_ctx* c, int nsubs) {
   return 0;
 }
 
-// Insertion order of a slice for the x4 kernels (SliceDesc::cols): along the
-// in-plane axis, DMS(1:3) (rows) or DMS(4:6) (columns), whose z component is
-// smaller, unless the context fixes one order.  Boxes up to 192 keep rows:
-// there a grid plane is at most 1.2 MB and the choice measured neutral
-// (192^3: 113.8k against 114.1k images/s of random orientations) or slower
-// (128^3: 260.1k against 262.4k), while at 256^3 it gains 5%.
-static short line_cols(const spi_ctx* c, const float* dms) {
-  if (c->line_order != 1) return c->line_order == 2 ? 1 : 0;
-  if (c->nx <= 192) return 0;
-  return std::fabs(dms[5]) < std::fabs(dms[2]) ? 1 : 0;
-}
-
 // Slice descriptors of nimg images: CANG of each angle triple (BUILDM1,
 // bp3f.f:1287), its products with the symmetry matrices (bp3f.f:460-466) and
 // the grid its half-set mask routes it to; image index a % chunk.  With slice
@@ -2507,8 +2328,7 @@ static void build_slices(const spi_ctx* c, const float* angles, const uint8_t* h
       SliceDesc& d = hs[(size_t)a * nsym + s];
       memcpy(d.dm, dms, 6 * sizeof(float));
       d.img = a % chunk;
-      d.grid = (short)g;
-      d.cols = line_cols(c, dms);
+      d.grid = g;
     }
   }
   if (!c->slice_order) return;
@@ -2746,6 +2566,7 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
 // runs on the first context's stream: while the call runs, the other
 // classes' contexts use that stream (their own are idle and restored after).
 namespace {
+constexpr int kMcMaxSizes = 8;
 struct StreamSwap {
   std::vector<spi_ctx*> ctxs;
   std::vector<cudaStream_t> saved;
@@ -2757,8 +2578,8 @@ struct StreamSwap {
 
 static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* const* imgs, const int* nimg,
                                 const float* const* angles, const uint8_t* const* half, int imgs_on_device) {
-  if (!ctxs || ncls < 1 || ncls > kMcMaxClass || !imgs || !nimg || !angles)
-    return fail(kInvalid, "spi_bp_insert_multi: %d classes (1..%d) or NULL arrays", ncls, kMcMaxClass);
+  if (!ctxs || ncls < 1 || ncls > kSlabMaxClass || !imgs || !nimg || !angles)
+    return fail(kInvalid, "spi_bp_insert_multi: %d classes (1..%d) or NULL arrays", ncls, kSlabMaxClass);
   spi_ctx* lead = ctxs[0];
   for (int k = 0; k < ncls; ++k) {
     spi_ctx* c = ctxs[k];
@@ -2771,22 +2592,16 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
     for (int j = 0; j < k; ++j)
       if (ctxs[j] == c) return fail(kInvalid, "spi_bp_insert_multi: class %d repeats a context", k);
   }
-  // one table per distinct box size
-  std::vector<int> tab_nx, cls_tab(ncls);
+  std::vector<int> sizes;   // at most kMcMaxSizes distinct boxes in one call
   for (int k = 0; k < ncls; ++k) {
-    auto it = std::find(tab_nx.begin(), tab_nx.end(), ctxs[k]->nx);
-    if (it == tab_nx.end()) {
-      if ((int)tab_nx.size() == kMcMaxTab)
-        return fail(kInvalid, "spi_bp_insert_multi: more than %d distinct box sizes", kMcMaxTab);
-      cls_tab[k] = (int)tab_nx.size();
-      tab_nx.push_back(ctxs[k]->nx);
-    } else {
-      cls_tab[k] = (int)(it - tab_nx.begin());
+    if (std::find(sizes.begin(), sizes.end(), ctxs[k]->nx) == sizes.end()) {
+      if ((int)sizes.size() == kMcMaxSizes)
+        return fail(kInvalid, "spi_bp_insert_multi: more than %d distinct box sizes", kMcMaxSizes);
+      sizes.push_back(ctxs[k]->nx);
     }
     if (!kb_window4_ok(ctxs[k]->kb))
       return fail(kInvalid, "spi_bp_insert_multi: the table of nx = %d is not a four-tap window", ctxs[k]->nx);
   }
-  const int ntab = (int)tab_nx.size();
   SPI_CUDA(cudaSetDevice(lead->device));
   StreamSwap swap;
   for (int k = 0; k < ncls; ++k) {
@@ -2803,49 +2618,12 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
     rounds = std::max(rounds, (nimg[k] + ctxs[k]->sub - 1) / ctxs[k]->sub);
     sl_off[k + 1] = sl_off[k] + (size_t)nimg[k] * ctxs[k]->nsym;
   }
-  // Everything the host copies during the call sits in one pinned buffer
-  // (copies from pageable memory would synchronise the stream every round):
-  // the slice descriptors of every class, one class table per round, the
-  // tables and their FLTB.
-  const size_t cls_bytes = sizeof(McClass) * kMcMaxClass;
-  const size_t h_sl = 0, h_cls = h_sl + sl_off[ncls] * sizeof(SliceDesc);
-  const size_t h_tab = h_cls + (size_t)std::max(rounds, 1) * cls_bytes;
-  SPI_TRY(lead->mc_host.ensure(h_tab + sizeof(float) * (5000 + 1) * kMcMaxTab));
-  SliceDesc* hs_all = reinterpret_cast<SliceDesc*>(lead->mc_host.as<char>() + h_sl);
-  McClass* hc_all = reinterpret_cast<McClass*>(lead->mc_host.as<char>() + h_cls);
-  float* ht = reinterpret_cast<float*>(lead->mc_host.as<char>() + h_tab);
-  float* hf = ht + 5000 * kMcMaxTab;
-  // launch parameters on the device: class table, then the tables and their FLTB
-  SPI_TRY(lead->mc_params.ensure(cls_bytes + sizeof(float) * (5000 + 1) * kMcMaxTab + sizeof(unsigned long long)));
-  auto* d_cls = lead->mc_params.as<McClass>();
-  float* d_tabs = reinterpret_cast<float*>(lead->mc_params.as<char>() + cls_bytes);
-  float* d_fl = d_tabs + 5000 * kMcMaxTab;
-  auto* d_work = reinterpret_cast<unsigned long long*>(d_fl + kMcMaxTab);
-  for (int t = 0; t < ntab; ++t)
-    for (int k = 0; k < ncls; ++k)
-      if (cls_tab[k] == t) {
-        memcpy(ht + (size_t)5000 * t, ctxs[k]->kb.tab, 5000 * sizeof(float));
-        hf[t] = ctxs[k]->kb.fltb;
-        break;
-      }
-  SPI_CUDA(cudaMemcpyAsync(d_tabs, ht, (size_t)5000 * ntab * sizeof(float), cudaMemcpyHostToDevice, st));
-  SPI_CUDA(cudaMemcpyAsync(d_fl, hf, ntab * sizeof(float), cudaMemcpyHostToDevice, st));
-  const size_t smem = (size_t)kMcTab * ntab * sizeof(float);
-  // every table must be zero from entry kMcTab - 1 on (checked above by kb_window4_ok: zero from 3331)
-  static_assert(kMcTab >= 3332, "the cut table must keep entries 0..3331");
-  {
-    static std::mutex mu;
-    static unsigned long long done = 0;
-    std::lock_guard<std::mutex> lk(mu);
-    const unsigned long long bit = 1ull << (lead->device & 63);
-    if (!(done & bit)) {
-      SPI_CUDA(cudaFuncSetAttribute(insert_mc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kMcTab * kMcMaxTab * sizeof(float))));
-      SPI_CUDA(cudaFuncSetAttribute(insert_mc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(kMcTab * kMcMaxTab * sizeof(float))));
-      done |= bit;
-    }
-  }
+  // The slice descriptors of every class sit in one pinned buffer (copies
+  // from pageable memory would synchronise the stream every round); the class
+  // table of a round goes with its launch.
+  SPI_TRY(lead->mc_host.ensure(std::max<size_t>(1, sl_off[ncls]) * sizeof(SliceDesc)));
+  SliceDesc* hs_all = lead->mc_host.as<SliceDesc>();
+  SPI_TRY(lead->workctr.ensure(sizeof(unsigned long long)));
   // per class: buffers (room for two FFT sub-batches: round r stages into
   // half r % 2 while round r - 1's insertion reads the other), slice
   // descriptors of all its images, staging constants
@@ -2881,9 +2659,8 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
   for (int k = 0; k < ncls; ++k) SPI_CUFFT(cufftSetStream(ctxs[k]->plan2d, s2));
   for (int r = 0; r < rounds; ++r) {
     const int h = r & 1;
-    McClass* hc = hc_all + (size_t)r * kMcMaxClass;
+    SlabArgs args{};
     int nc = 0;
-    long long items = 0;
     if (r >= 2) SPI_CUDA(cudaStreamWaitEvent(s2, lead->ev_done[h], 0));   // round r - 2 read this half
     for (int k = 0; k < ncls; ++k) {
       spi_ctx* c = ctxs[k];
@@ -2923,36 +2700,17 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
       SliceDesc* dsl = c->slices.as<SliceDesc>() + hoff * c->nsym;
       SPI_CUDA(cudaMemcpyAsync(dsl, hs_all + sl_off[k] + (size_t)a0 * c->nsym, nsl * sizeof(SliceDesc),
                                cudaMemcpyHostToDevice, s2));
-      McClass m{};
-      m.spec = c->bf16 ? (const void*)(reinterpret_cast<__nv_bfloat162*>(c->spectra.p) + hoff * plane)
-                       : (const void*)(c->spectra.as<float2>() + hoff * plane);
-      m.slices = dsl;
-      m.g0 = insert_target(c, 0);
-      m.g1 = insert_target(c, c->ngrids == 2 ? 1 : 0);
-      m.item0 = items;
-      m.nx = nx;
-      m.nslices = (int)nsl;
-      m.tab = cls_tab[k];
-      hc[nc++] = m;
-      items += (long long)nsl * n;
+      const void* spec = c->bf16 ? (const void*)(reinterpret_cast<__nv_bfloat162*>(c->spectra.p) + hoff * plane)
+                                 : (const void*)(c->spectra.as<float2>() + hoff * plane);
+      args.cls[nc++] = slab_class(c, spec, dsl, (int)nsl, insert_target(c, 0), insert_target(c, c->ngrids == 2 ? 1 : 0));
     }
     SPI_CUDA(cudaEventRecord(lead->ev_ready[h], s2));
     if (nc == 0) continue;
     SPI_CUDA(cudaStreamWaitEvent(st, lead->ev_ready[h], 0));
-    SPI_CUDA(cudaMemcpyAsync(d_cls, hc, nc * sizeof(McClass), cudaMemcpyHostToDevice, st));
-    SPI_CUDA(cudaMemsetAsync(d_work, 0, sizeof(unsigned long long), st));
-    int per_sm = 1;
-    if (lead->bf16)
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, insert_mc_kernel<true>, 512, smem);
-    else
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, insert_mc_kernel<false>, 512, smem);
-    const int blocks = lead->sm_count * std::max(1, std::min(per_sm, env_int("SPI_MC_BLOCKS_PER_SM", 2)));
+    args.ncls = nc;
+    args.nitems = slab_items(lead->sm_count, args.cls, nc);
     int ev = lead->phase_begin(2, st);
-    if (lead->bf16)
-      insert_mc_kernel<true><<<blocks, 512, smem, st>>>(d_cls, nc, items, d_tabs, d_fl, ntab, d_work);
-    else
-      insert_mc_kernel<false><<<blocks, 512, smem, st>>>(d_cls, nc, items, d_tabs, d_fl, ntab, d_work);
-    SPI_TRY(check_kernel("insert_mc_kernel"));
+    SPI_TRY(launch_slab(lead, args, lead->bf16, lead->workctr.as<unsigned long long>(), env_int("SPI_MC_BLOCKS_PER_SM", kSlabBlocks), st));
     lead->phase_end(ev);
     lead->count();
     SPI_CUDA(cudaEventRecord(lead->ev_done[h], st));
@@ -3029,8 +2787,7 @@ static int bp_autotune_impl(spi_ctx* c, int force) {
       SliceDesc& d = hs[(size_t)a * nsym + sy];
       memcpy(d.dm, dms, 6 * sizeof(float));
       d.img = a;
-      d.grid = (c->ngrids == 2) ? (short)(a & 1) : 0;
-      d.cols = line_cols(c, dms);
+      d.grid = (c->ngrids == 2) ? (a & 1) : 0;
     }
   }
   SPI_CUDA(cudaMemcpyAsync(c->slices.p, hs, nsl * sizeof(SliceDesc), cudaMemcpyHostToDevice, c->stream));
@@ -3038,7 +2795,9 @@ static int bp_autotune_impl(spi_ctx* c, int force) {
   SPI_CUDA(cudaMemsetAsync(c->spectra.p, 0, (size_t)sample * plane * (c->bf16 ? 4 : 8), c->stream));
   float4* g1 = insert_target(c, c->ngrids == 2 ? 1 : 0);
   const int modes[2] = {kb_window4_ok(c->kb) ? 3 : 2, 2};
-  const int shapes[5][2] = {{256, 2}, {256, 3}, {512, 2}, {128, 4}, {512, 1}};
+  // threads and CTAs per SM; the column kernel has its own CTA size (kSlabThreads consumers) and two shapes
+  const int shapes[2][5][2] = {{{kSlabThreads, kSlabBlocks}, {kSlabThreads, kSlabBlocks - 1}, {0, 0}, {0, 0}, {0, 0}},
+                               {{256, 2}, {256, 3}, {512, 2}, {128, 4}, {512, 1}}};
   cudaEvent_t e0, e1;
   SPI_CUDA(cudaEventCreate(&e0));
   if (cudaEventCreate(&e1) != cudaSuccess) {
@@ -3059,8 +2818,10 @@ static int bp_autotune_impl(spi_ctx* c, int force) {
       if (mi == 1 && modes[0] == modes[1]) break;
       for (int si = 0; si < 5; ++si) {
         c->insert_mode = modes[mi];
-        c->insert_threads = shapes[si][0];
-        c->insert_blocks_per_sm = shapes[si][1];
+        const int* shape = shapes[modes[mi] == 3 ? 0 : 1][si];
+        if (shape[0] == 0) break;
+        c->insert_threads = shape[0];
+        c->insert_blocks_per_sm = shape[1];
         if ((st = launch_insert(c, c->slices.as<SliceDesc>(), (int)nsl, g1))) break;   // warm-up
         cudaEventRecord(e0, c->stream);
         for (int r = 0; r < 2 && !st; ++r) st = launch_insert(c, c->slices.as<SliceDesc>(), (int)nsl, g1);
@@ -3073,7 +2834,10 @@ static int bp_autotune_impl(spi_ctx* c, int force) {
     }
   for (int mi = 0; mi < 2; ++mi)
     for (int si = 0; si < 5; ++si)
-      if (tmin[mi][si] < best.ms) best = TuneVal{modes[mi], shapes[si][0], shapes[si][1], tmin[mi][si]};
+      if (tmin[mi][si] < best.ms) {
+        const int* shape = shapes[modes[mi] == 3 ? 0 : 1][si];
+        best = TuneVal{modes[mi], shape[0], shape[1], tmin[mi][si]};
+      }
   c->timing = timing;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);

@@ -20,9 +20,8 @@ struct spi_ctx {
   float tuned_ms = 0.0f;              // autotuner: time of the chosen launch on its sample
   int bf16 = 0;
   int insert_mode = 3;                // 0 = tile-privatised, 1 = direct per-tap atomics, 2 = five x-tap lanes,
-                                      // 3 = four lanes over the nonzero tap window
+                                      // 3 = voxel columns, taps summed in registers
   int slice_order = 1;                // 1 = order slices of a chunk by plane normal
-  int line_order = 1;                 // x4 insertion order: 0 rows, 2 columns, 1 per slice (SliceDesc::cols)
   int insert_seg_map = 0;             // 1 = warps take 32-pixel row segments, 0 = whole rows
   int insert_threads = 256;           // threads per insert block
   int insert_blocks_per_sm = 0;       // 0 = as many as fit
@@ -62,8 +61,7 @@ struct spi_ctx {
   spi::DevBuf spec_tmp;               // float2 [sub][n][nx+1] (BF16 mode FFT output)
   spi::DevBuf slices;                 // SliceDesc [chunk * nsym]
   spi::DevBuf workctr;                // u64 row counter of the running insert launch
-  spi::DevBuf mc_params;              // multi-class insertion: class table + tables of the launch
-  spi::HostBuf mc_host;               // multi-class insertion: pinned descriptors, class tables, tables
+  spi::HostBuf mc_host;               // multi-class insertion: pinned slice descriptors
   spi::DevBuf cplx;                   // float2 [n][n][nx+1] (inverse FFT input)
   spi::DevBuf real3;                  // float [n][n][n]
   spi::DevBuf wkb;                    // float[(nx/2)^2 + 1]

@@ -1,0 +1,181 @@
+// CPU check of the column insertion's geometry (spider_b200/csrc/slab_geom.h):
+// for each box size and rotation the taps that the columns of every tile find
+// are compared, voxel by voxel, with ONELINE's own walk over the pixels
+// (restated here from oneline.f:38-200).
+//
+//   slab_check NX SEED COUNT   ->  one line per rotation:
+//   kind banks max_rows max_pixels taps_direct taps_columns bad
+// `bad` counts voxels whose set of (pixel, weight bits) differs, taps outside
+// their column's voxel range, tiles over the capacity, and pixel rows or spans
+// that do not cover a tap.
+#include <cstdint>
+#include <cstdio>
+#include <cstdlib>
+#include <cstring>
+#include <map>
+#include <random>
+#include <utility>
+#include <vector>
+
+#include "../spider_b200/csrc/slab_geom.h"
+
+using namespace spi;
+
+static std::vector<float> g_tab;
+static float g_fltb;
+static const int kLast = 3331;
+
+static float tap(float c, int k) { return g_tab[slab_tab_index(c, k, g_fltb, kLast)]; }
+
+// key of a tap: voxel and pixel (of the full disc), value: bits of the weight
+typedef std::map<std::pair<long long, int>, std::vector<uint32_t>> Taps;
+
+static long long vox(int x, int y, int z, int nx) {
+  const int N = 2 * nx;
+  const int iy = y >= 0 ? y : N + y, iz = z >= 0 ? z : N + z;
+  return ((long long)iz * N + iy) * (nx + 1) + x;
+}
+
+static uint32_t wbits(float wx, float wy, float wz) {
+  const float w = wx * (wy * wz);
+  uint32_t b;
+  memcpy(&b, &w, 4);
+  return b;
+}
+
+// ONELINE over the half disc; pixel id of the canonical pixel and its mate
+static long long direct(const float* dm, int nx, Taps& t) {
+  const int N = 2 * nx, W = 2 * nx + 1;
+  long long n = 0;
+  for (int J = -nx + 1; J <= nx; ++J)
+    for (int I = 0; I <= nx; ++I) {
+      if (I * I + J * J >= nx * nx || (I == 0 && J < 0)) continue;
+      float c[3];
+      for (int a = 0; a < 3; ++a) {
+        const float p = (float)I * dm[a], q = (float)J * dm[a + 3];
+        c[a] = p + q;
+      }
+      int s = 1;
+      if (c[0] < 0) { for (float& v : c) v = -v; s = -1; }
+      int k[3];
+      for (int a = 0; a < 3; ++a) { const float h = c[a] + 0.5f; k[a] = (int)(h + (float)N) - N; }
+      if (!(k[0] <= nx - 3 && k[1] >= -nx + 4 && k[1] <= nx - 3 && k[2] >= -nx + 4 && k[2] <= nx - 3)) continue;
+      for (int lz = -2; lz <= 2; ++lz)
+        for (int ly = -2; ly <= 2; ++ly)
+          for (int lx = -2; lx <= 2; ++lx) {
+            const int x = k[0] + lx, y = k[1] + ly, z = k[2] + lz;
+            const float wx = tap(c[0], x), wy = tap(c[1], y), wz = tap(c[2], z);
+            if (wx * (wy * wz) == 0.0f) continue;
+            // pixel that lies where the tap lands: the canonical one, or its mate for a reflected tap
+            const int sg = x < 0 ? -s : s;
+            const int id = (sg * J + nx) * W + sg * I + nx;
+            t[{x < 0 ? vox(-x, -y, -z, nx) : vox(x, y, z, nx), id}].push_back(wbits(wx, wy, wz));
+            ++n;
+          }
+    }
+  return n;
+}
+
+int main(int argc, char** argv) {
+  const int nx = atoi(argv[1]), count = atoi(argv[3]);
+  std::mt19937 rng(atoi(argv[2]));
+  // a stand-in for FILLBESSIL's table with its support: nonzero up to 1.8, zero beyond
+  g_fltb = 4999.0f / 3.0f;
+  g_tab.assign(5000, 0.0f);
+  for (int i = 0; i < 5000; ++i)
+    if ((float)i / g_fltb <= 1.8f) g_tab[i] = 1.0f + (float)(5000 - i) * 1.37e-4f;
+  std::uniform_real_distribution<double> U(0.0, 1.0);
+  for (int q = 0; q < count; ++q) {
+    double ps = 2 * M_PI * U(rng), th = acos(1 - 2 * U(rng)), ph = 2 * M_PI * U(rng);
+    // the rotations where the geometry degenerates come first: axes, diagonals, planes of 45 degrees
+    const double sp[12][3] = {{0, 0, 0}, {0, M_PI / 2, 0}, {0, M_PI / 2, M_PI / 2}, {M_PI / 4, 0, 0},
+                              {0, M_PI / 4, 0}, {M_PI / 4, acos(1 / sqrt(3.0)), M_PI / 4}, {0, M_PI, 0},
+                              {M_PI / 2, M_PI / 2, M_PI / 4}, {0.3, M_PI / 2, M_PI / 4}, {M_PI, acos(1 / sqrt(3.0)), -M_PI / 4},
+                              {0, acos(1 / sqrt(3.0)), M_PI / 4}, {1.1, M_PI / 4, M_PI / 2}};
+    if (q < 12) { ps = sp[q][0]; th = sp[q][1]; ph = sp[q][2]; }
+    const double cp = cos(ps), s_p = sin(ps), ct = cos(th), st = sin(th), cf = cos(ph), sf = sin(ph);
+    const float dm[6] = {(float)(cf * ct * cp - sf * s_p), (float)(sf * ct * cp + cf * s_p), (float)(-st * cp),
+                         (float)(-cf * ct * s_p - sf * cp), (float)(-sf * ct * s_p + cf * cp), (float)(st * s_p)};
+    Taps A, B;
+    long long na = direct(dm, nx, A), nb = 0, bad = 0;
+    SlabFrame f;
+    int rows = 0, pixels = 0, banks = 0;
+    if (!slab_frame(dm, f)) { printf("noframe\n"); continue; }
+    banks = slab_banks(f);
+    const int nu = banks == 2 ? 2 : 1;   // columns along u of a thread's block
+    const int W = 2 * nx + 1;
+    const int ntu = f.d == 0 ? (2 * nx + kSlabTile - 1) / kSlabTile : (nx + kSlabTile - 1) / kSlabTile;
+    const int ntv = (2 * nx + kSlabTile - 1) / kSlabTile;
+    for (int tv = 0; tv < ntv; ++tv)
+      for (int tu = 0; tu < ntu; ++tu) {
+        const int u0 = (f.d == 0 ? -nx : 0) + kSlabTile * tu, v0 = -nx + kSlabTile * tv;
+        if (!slab_tile_live(f, u0, v0, nx)) continue;
+        int jlo, nr;
+        slab_tile_rows(f, u0, v0, nx, jlo, nr);
+        std::vector<int> lo(nr), hi(nr);
+        int np = 0;
+        for (int r = 0; r < nr; ++r) {
+          slab_tile_span(f, u0, v0, nx, jlo + r, lo[r], hi[r]);
+          np += hi[r] >= lo[r] ? hi[r] - lo[r] + 1 : 0;
+        }
+        if (nr > rows) rows = nr;
+        if (np > pixels) pixels = np;
+        if (nr >= kSlabRows || np > kSlabPix) ++bad;
+        for (int du = 0; du < kSlabTile; du += nu)
+          for (int dv = 0; dv < kSlabTile; dv += 2) {   // a block of columns at a time, as the kernel's threads take them
+            int r0, r1;
+            const float u = (float)(u0 + du), v = (float)(v0 + dv);
+            slab_block_rows(f, u, v, nu, 2, jlo, nr, r0, r1);
+            for (int r = r0; r <= r1; ++r) {
+              float fl, fh;
+              slab_span(f, u + 0.5f * (nu - 1), v + 0.5f, kSlabR + 0.5f * (nu - 1), kSlabR + 0.5f, jlo + r, fl, fh);
+              const int i0 = slab_ceil(fmaxf(fl, (float)lo[r])), i1 = slab_floor(fminf(fh, (float)hi[r]));
+              for (int I = i0; I <= i1; ++I) {
+                const SlabPix p = slab_pixel(f, I, jlo + r);
+                if (!slab_inside(f, p, I, jlo + r, nx)) continue;
+                const int au = f.d == 0 ? 1 : 0, av = f.d == 2 ? 1 : 2, aw = f.d;
+                float pos[3];
+                pos[au] = p.u;
+                pos[av] = p.v;
+                pos[aw] = p.w;
+                for (int c = 0; c < 2 * nu; ++c) {
+                  int k[3];
+                  k[au] = u0 + du + c / 2;
+                  k[av] = v0 + dv + c % 2;
+                  // the kernel's table has no bound on the index
+                  if (slab_tab_index(p.u, k[au], g_fltb, 9999) >= kSlabTab || slab_tab_index(p.v, k[av], g_fltb, 9999) >= kSlabTab) ++bad;
+                  const int base = slab_col_base(f, (float)k[au], (float)k[av]);
+                  for (int l = 0; l < 4; ++l) {
+                    k[aw] = slab_first(p.w) + l;
+                    const float wx = tap(pos[0], k[0]), wy = tap(pos[1], k[1]), wz = tap(pos[2], k[2]);
+                    if (wx * (wy * wz) == 0.0f) continue;
+                    if (k[0] < 0 || (k[0] == 0 && !p.canon)) continue;
+                    // the residue must give the voxel back
+                    const int off = slab_residue(k[aw], banks) - slab_residue(base, banks);
+                    if (base + (off < 0 ? off + 4 * banks : off) != k[aw]) ++bad;
+                    B[{vox(k[0], k[1], k[2], nx), (jlo + r + nx) * W + I + nx}].push_back(wbits(wx, wy, wz));
+                    ++nb;
+                  }
+                }
+              }
+            }
+          }
+      }
+    // the origin's reflected taps (it is its own mate)
+    const int id0 = nx * W + nx;
+    for (int x = 1; x <= 1; ++x)
+      for (int y = -1; y <= 1; ++y)
+        for (int z = -1; z <= 1; ++z) {
+          B[{vox(x, -y, -z, nx), id0}].push_back(wbits(tap(0, x), tap(0, y), tap(0, z)));
+          ++nb;
+        }
+    for (auto& e : A) {
+      auto it = B.find(e.first);
+      if (it == B.end() || it->second != e.second) ++bad;
+    }
+    for (auto& e : B)
+      if (!A.count(e.first)) ++bad;
+    printf("%d %d %d %d %lld %lld %lld\n", f.d, banks, rows, pixels, na, nb, bad);
+  }
+  return 0;
+}

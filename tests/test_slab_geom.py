@@ -1,0 +1,30 @@
+"""The column insertion's geometry on the CPU: every tap of ONELINE's walk over
+the pixels is found by exactly one voxel column, with the same weight bits."""
+import os
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("slab") / "slab_check")
+    subprocess.run(["g++", "-O2", "-std=c++17", "-ffp-contract=off", "-o", exe, os.path.join(HERE, "slab_check.cpp")],
+                   check=True)
+    return exe
+
+
+@pytest.mark.parametrize("nx,count", [(8, 40), (9, 30), (15, 30), (16, 30), (17, 30), (33, 24), (48, 16)])
+def test_columns_find_every_tap(check, nx, count):
+    """Smallest box, odd boxes, boxes around one and two tiles; the first twelve
+    rotations are the degenerate ones (axes, diagonals, 45 degree planes)."""
+    out = subprocess.run([check, str(nx), "5", str(count)], check=True, capture_output=True, text=True).stdout
+    rows = [tuple(map(int, line.split())) for line in out.splitlines()]
+    assert len(rows) == count
+    for d, banks, nrows, npix, direct, columns, bad in rows:
+        assert bad == 0 and direct == columns > 0
+        assert nrows <= 47 and npix <= 654
+    assert {r[0] for r in rows} == {0, 1, 2}        # every dominant axis
+    assert {r[1] for r in rows} == {2, 3}           # shallow and steep slices
