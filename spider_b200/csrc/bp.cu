@@ -1671,11 +1671,11 @@ void bp_release(spi_ctx* c) {
   c->volbuf.release();
   c->symtmp.release();
   c->hslices.release();
-  if (c->plan2d) cufftDestroy(c->plan2d);
+  for (auto& p : c->plans2d) cufftDestroy(p.plan);
+  c->plans2d.clear();
   if (c->plan3d) cufftDestroy(c->plan3d);
-  c->plan2d = 0;
   c->plan3d = 0;
-  c->plan2d_n = c->plan2d_batch = c->plan3d_n = 0;
+  c->plan3d_n = 0;
   c->nx = c->n = c->ngrids = 0;
   c->pending_sym0[0] = c->pending_sym0[1] = false;
   c->merged = false;
@@ -2116,28 +2116,74 @@ static int ensure_fft_twiddles(spi_ctx* c) {
   return 0;
 }
 
-static int ensure_chunk_buffers(spi_ctx* c) {
+// Images a transform of m valid ones takes.  cuFFT plans have a fixed batch:
+// a call's last, shorter sub-batch takes the next of 16, 24, 32, 48, ... (at
+// most a third of padding, and few plans per context) instead of a whole
+// sub-batch of up to 1 GB (300 images of 147^2 used to transform 3,106: 2.6 ms
+// against 0.3 ms).  The own R2C transforms the valid images only.
+static int fft_batch(const spi_ctx* c, int m) {
+  if (c->fft_own) return m;
+  if (m >= c->sub) return c->sub;
+  int b = 16;
+  while (b < m) {
+    if (b + b / 2 >= m) {
+      b += b / 2;
+      break;
+    }
+    b *= 2;
+  }
+  return std::min(b, c->sub);
+}
+
+// The R2C plan of `batch` images of the open reconstruction's size; the
+// least recently used of kPlans2d makes room for a new one.
+static int plan2d_of(spi_ctx* c, int batch, cufftHandle* out) {
+  constexpr size_t kPlans2d = 4;
+  auto& v = c->plans2d;
+  for (size_t i = 0; i < v.size(); ++i)
+    if (v[i].n == c->n && v[i].batch == batch) {
+      std::rotate(v.begin(), v.begin() + i, v.begin() + i + 1);
+      *out = v[0].plan;
+      return 0;
+    }
+  const int n = c->n;
+  int dims[2] = {n, n};
+  cufftHandle h = 0;
+  SPI_CUFFT(cufftPlanMany(&h, 2, dims, nullptr, 1, n * n, nullptr, 1, n * (n / 2 + 1), CUFFT_R2C, batch));
+  if (v.size() == kPlans2d) {
+    cufftDestroy(v.back().plan);
+    v.pop_back();
+  }
+  v.insert(v.begin(), spi_ctx::Plan2d{h, n, batch});
+  *out = h;
+  return 0;
+}
+static int exec_r2c(spi_ctx* c, cudaStream_t st, int batch, float* in, float2* out) {
+  cufftHandle h = 0;
+  SPI_TRY(plan2d_of(c, batch, &h));
+  SPI_CUFFT(cufftSetStream(h, st));
+  SPI_CUFFT(cufftExecR2C(h, in, reinterpret_cast<cufftComplex*>(out)));
+  return 0;
+}
+
+// Staging buffers for chunks of at most `images` images (<= c->chunk), whose
+// spectra are transformed in sub-batches from the chunk's start
+static int ensure_chunk_buffers(spi_ctx* c, int images, bool host_images) {
   const int nx = c->nx, n = c->n;
   if (c->fft_own) SPI_TRY(ensure_fft_twiddles(c));
-  SPI_TRY(c->imgs.ensure((size_t)c->chunk * nx * nx * sizeof(float)));
-  SPI_TRY(c->padded.ensure((size_t)c->sub * n * n * sizeof(float)));
+  const int subs = images / c->sub, rest = images % c->sub;
+  const size_t rows = (size_t)subs * c->sub + (rest ? fft_batch(c, rest) : 0);   // spectra the transforms write
+  const size_t batch = (size_t)fft_batch(c, std::min(images, c->sub));
+  if (host_images) SPI_TRY(c->imgs.ensure((size_t)images * nx * nx * sizeof(float)));
+  SPI_TRY(c->padded.ensure(batch * n * n * sizeof(float)));
   const size_t plane = (size_t)n * (nx + 1);
   if (c->bf16) {
-    SPI_TRY(c->spectra.ensure((size_t)c->chunk * plane * sizeof(__nv_bfloat162)));
-    SPI_TRY(c->spec_tmp.ensure((size_t)c->sub * plane * sizeof(float2)));
+    SPI_TRY(c->spectra.ensure((size_t)images * plane * sizeof(__nv_bfloat162)));
+    SPI_TRY(c->spec_tmp.ensure(batch * plane * sizeof(float2)));
   } else {
-    SPI_TRY(c->spectra.ensure((size_t)c->chunk * plane * sizeof(float2)));
+    SPI_TRY(c->spectra.ensure(rows * plane * sizeof(float2)));
   }
-  SPI_TRY(c->slices.ensure((size_t)c->chunk * c->nsym * sizeof(SliceDesc)));
-  if (c->plan2d == 0 || c->plan2d_n != n || c->plan2d_batch != c->sub) {
-    if (c->plan2d) cufftDestroy(c->plan2d);
-    c->plan2d = 0;
-    int dims[2] = {n, n};
-    SPI_CUFFT(cufftPlanMany(&c->plan2d, 2, dims, nullptr, 1, n * n, nullptr, 1, n * (n / 2 + 1), CUFFT_R2C, c->sub));
-    SPI_CUFFT(cufftSetStream(c->plan2d, c->stream));
-    c->plan2d_n = n;
-    c->plan2d_batch = c->sub;
-  }
+  SPI_TRY(c->slices.ensure((size_t)images * c->nsym * sizeof(SliceDesc)));
   return 0;
 }
 
@@ -2370,7 +2416,8 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
   if (c->merged) return fail(kInvalid, "spi_bp_insert: images cannot follow spi_bp_partial_add");
   if (nimg == 0) return 0;
   SPI_CUDA(cudaSetDevice(c->device));
-  SPI_TRY(ensure_chunk_buffers(c));
+  const int most = std::min(nimg, c->chunk);   // images of the call's largest chunk
+  SPI_TRY(ensure_chunk_buffers(c, most, !imgs_on_device));
   c->inserted = true;
   const int nx = c->nx, n = c->n, nsym = c->nsym;
   // slice descriptors for the whole call (host, pinned)
@@ -2428,8 +2475,8 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
         rprm[a] = RtsqParm{std::cos(theta), std::sin(theta), modulo(inplane[3 * a + 1]), modulo(inplane[3 * a + 2])};
       }
     }
-    SPI_TRY(c->imgs2.ensure((size_t)c->chunk * nx * nx * sizeof(float)));
-    SPI_TRY(c->rtsq_prm.ensure((size_t)c->chunk * sizeof(RtsqParm)));
+    SPI_TRY(c->imgs2.ensure((size_t)most * nx * nx * sizeof(float)));
+    SPI_TRY(c->rtsq_prm.ensure((size_t)most * sizeof(RtsqParm)));
   }
   // Copy pipeline.  With host images, the copy stream uploads the chunk in
   // pieces of `up` images (<= ~64 MB) and records ev_ready per piece; the
@@ -2451,7 +2498,6 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
     SPI_CUDA(cudaEventRecord(c->ev_fork, c->stream));
     SPI_CUDA(cudaStreamWaitEvent(cs, c->ev_fork, 0));
   }
-  SPI_CUFFT(cufftSetStream(c->plan2d, c->stream));
   std::vector<char> done_valid(nsubs, 0);
   float4* g1 = insert_target(c, c->ngrids == 2 ? 1 : 0);
   for (int a0 = 0; a0 < nimg; a0 += c->chunk) {
@@ -2513,7 +2559,7 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
                                 c->padded.as<float2>() + (size_t)(p0 - b0) * n * n / 2));
         } else {
           // the last piece also zero-pads the unused tail of the FFT batch
-          const int blocks = last ? c->sub - (p0 - b0) : np;
+          const int blocks = last ? fft_batch(c, nvalid) - (p0 - b0) : np;
           const int parts = std::max(1, std::min(8, (4 * c->sm_count + blocks - 1) / std::max(blocks, 1)));
           stage_kernel<<<dim3(blocks, parts), 256, 0, c->stream>>>(src, nx, n, ip, np, klp,
                                                                    c->padded.as<float>() + (size_t)(p0 - b0) * n * n);
@@ -2530,7 +2576,7 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
         SPI_TRY(launch_colfft(c, c->stream, c->padded.as<float2>(), nvalid, fout));
         c->count();
       } else {
-        SPI_CUFFT(cufftExecR2C(c->plan2d, c->padded.as<cufftReal>(), reinterpret_cast<cufftComplex*>(fout)));
+        SPI_TRY(exec_r2c(c, c->stream, fft_batch(c, nvalid), c->padded.as<float>(), fout));
       }
       c->phase_end(ev);
       if (c->bf16) {
@@ -2628,16 +2674,18 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
   // half r % 2 while round r - 1's insertion reads the other), slice
   // descriptors of all its images, staging constants
   std::vector<double> klp(ncls);
+  std::vector<size_t> half_rows(ncls, 0);   // images of one half
   for (int k = 0; k < ncls; ++k) {
     spi_ctx* c = ctxs[k];
-    SPI_TRY(ensure_chunk_buffers(c));
-    const size_t two = (size_t)std::max(c->chunk, 2 * c->sub);
+    if (nimg[k] == 0) continue;
+    const int most = std::min(c->sub, nimg[k]);
+    half_rows[k] = (size_t)fft_batch(c, most);
+    SPI_TRY(ensure_chunk_buffers(c, most, false));
     const size_t plane = (size_t)c->n * (c->nx + 1);
-    SPI_TRY(c->spectra.ensure(two * plane * (c->bf16 ? sizeof(__nv_bfloat162) : sizeof(float2))));
-    SPI_TRY(c->slices.ensure(two * c->nsym * sizeof(SliceDesc)));
-    if (!imgs_on_device) SPI_TRY(c->imgs.ensure(two * c->nx * c->nx * sizeof(float)));
-    if (nimg[k] > 0)
-      build_slices(c, angles[k], half ? half[k] : nullptr, nimg[k], c->sub, c->sub, c->sub, c->sub, hs_all + sl_off[k]);
+    SPI_TRY(c->spectra.ensure(2 * half_rows[k] * plane * (c->bf16 ? sizeof(__nv_bfloat162) : sizeof(float2))));
+    SPI_TRY(c->slices.ensure(2 * half_rows[k] * c->nsym * sizeof(SliceDesc)));
+    if (!imgs_on_device) SPI_TRY(c->imgs.ensure(2 * half_rows[k] * c->nx * c->nx * sizeof(float)));
+    build_slices(c, angles[k], half ? half[k] : nullptr, nimg[k], c->sub, c->sub, c->sub, c->sub, hs_all + sl_off[k]);
     const int nx = c->nx;
     int cnt = 0;
     const float rr = (float)(nx / 2) * (float)(nx / 2);
@@ -2648,7 +2696,7 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
         if (t * t + t2 * t2 > rr) ++cnt;
       }
     klp[k] = (double)(float)cnt;
-    if (nimg[k] > 0) c->inserted = true;
+    c->inserted = true;
   }
   // rounds: every class stages its next FFT sub-batch on the staging stream,
   // then one launch on the compute stream inserts them all
@@ -2656,7 +2704,6 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
   SPI_TRY(ensure_pipeline_events(lead, 2));   // ev_ready[h]: half h staged; ev_done[h]: half h inserted
   SPI_CUDA(cudaEventRecord(lead->ev_fork, st));
   SPI_CUDA(cudaStreamWaitEvent(s2, lead->ev_fork, 0));
-  for (int k = 0; k < ncls; ++k) SPI_CUFFT(cufftSetStream(ctxs[k]->plan2d, s2));
   for (int r = 0; r < rounds; ++r) {
     const int h = r & 1;
     SlabArgs args{};
@@ -2668,7 +2715,7 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
       const int a0 = r * c->sub, nb = std::min(c->sub, nimg[k] - a0);
       if (nb <= 0) continue;
       const size_t plane = (size_t)n * (nx + 1);
-      const size_t hoff = (size_t)h * c->sub;   // first image of this half
+      const size_t hoff = (size_t)h * half_rows[k];   // first image of this half
       const float* src = imgs[k] + (size_t)a0 * nx * nx;
       if (!imgs_on_device) {
         float* dst = c->imgs.as<float>() + hoff * nx * nx;
@@ -2676,7 +2723,8 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
         src = dst;
       }
       const int ip = (n - nx) / 2 + nx % 2;
-      const int parts = std::max(1, std::min(8, (4 * c->sm_count + c->sub - 1) / c->sub));
+      const int batch = fft_batch(c, nb);
+      const int parts = std::max(1, std::min(8, (4 * c->sm_count + batch - 1) / batch));
       float2* fout = c->bf16 ? c->spec_tmp.as<float2>() : c->spectra.as<float2>() + hoff * plane;
       if (c->fft_own) {   // the own R2C (the class's box takes the same default as spi_bp_insert)
         const int rparts = std::max(1, std::min(8, (4 * c->sm_count + nb - 1) / std::max(nb, 1)));
@@ -2684,10 +2732,10 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
         SPI_TRY(launch_colfft(c, s2, c->padded.as<float2>(), nb, fout));
         c->count(2);
       } else {
-        stage_kernel<<<dim3(c->sub, parts), 256, 0, s2>>>(src, nx, n, ip, nb, klp[k], c->padded.as<float>());
+        stage_kernel<<<dim3(batch, parts), 256, 0, s2>>>(src, nx, n, ip, nb, klp[k], c->padded.as<float>());
         SPI_TRY(check_kernel("stage_kernel"));
         c->count();
-        SPI_CUFFT(cufftExecR2C(c->plan2d, c->padded.as<cufftReal>(), reinterpret_cast<cufftComplex*>(fout)));
+        SPI_TRY(exec_r2c(c, s2, batch, c->padded.as<float>(), fout));
       }
       if (c->bf16) {
         const size_t cntv = (size_t)nb * plane;
@@ -2769,9 +2817,9 @@ static int bp_autotune_impl(spi_ctx* c, int force) {
       return 0;
     }
   }
-  SPI_TRY(ensure_chunk_buffers(c));
   const int nx = c->nx, nsym = c->nsym;
   const int sample = std::min(c->sub, 512);
+  SPI_TRY(ensure_chunk_buffers(c, sample, false));
   const size_t nsl = (size_t)sample * nsym;
   SPI_TRY(c->hslices.ensure(nsl * sizeof(SliceDesc)));
   SliceDesc* hs = c->hslices.as<SliceDesc>();

@@ -69,8 +69,8 @@ struct spi_ctx {
   spi::DevBuf volbuf;                 // float [nx^3] (finish output staging)
   spi::DevBuf symtmp;                 // float [nx^3] + symmetry matrices (SYMVOL input)
   spi::HostBuf hslices;
-  cufftHandle plan2d = 0;
-  int plan2d_n = 0, plan2d_batch = 0;
+  struct Plan2d { cufftHandle plan; int n, batch; };
+  std::vector<Plan2d> plans2d;        // batched R2C plans, most recently used first
   int fft_own = 0;                    // 1 = the library's own two-pass R2C (power-of-two n), 0 = cuFFT
   spi::DevBuf fft_tw;                 // float2 W_n^t, t < n/2 (FP64-computed twiddles of the own R2C)
   cufftHandle plan3d = 0;
