@@ -311,6 +311,15 @@ int spi_fslice_normal(const spi_fslice_plan* plan, const float* grid_in, float l
  * that many digits. */
 int spi_fslice_normal64(const spi_fslice_plan* plan, const double* grid_in, double lam, double* grid_out,
                         void* stream);
+/* The same normal operator (fp64 = 0: float2 grids, 1: double2) through a
+ * caller's workspace: the slices of E go to `ws`, as many at a time as it
+ * holds, and E^T adds them back.  About 1.5 to 2 times as fast as the two calls
+ * above, which keep no slices.  ws: device memory, 16-byte aligned, at least one
+ * slice (2nx * (nx+1) complex values) and 8 bytes per slice of the plan;
+ * spi_fslice_normal_ws_bytes gives a good size.  Not shared between calls that may run at the same time. */
+int spi_fslice_normal_ws_bytes(const spi_fslice_plan* plan, int fp64, long long* bytes);
+int spi_fslice_normal_ws(const spi_fslice_plan* plan, const void* grid_in, double lam, void* grid_out, int fp64,
+                         void* ws, long long ws_bytes, void* stream);
 /* slices = E grid on FP64 arrays (FP64 sums of the same taps; an exact
  * reference for gradient checks of the FP32 extraction). */
 int spi_fslice_forward64(const spi_fslice_plan* plan, const double* grid, double* slices, void* stream);

@@ -66,6 +66,9 @@ SIGNATURES = [
     ("spi_fslice_adjoint", ctypes.c_int, [_vp, _vp, _vp, _vp]),
     ("spi_fslice_normal", ctypes.c_int, [_vp, _vp, ctypes.c_float, _vp, _vp]),
     ("spi_fslice_normal64", ctypes.c_int, [_vp, _vp, ctypes.c_double, _vp, _vp]),
+    ("spi_fslice_normal_ws_bytes", ctypes.c_int, [_vp, ctypes.c_int, ctypes.POINTER(ctypes.c_longlong)]),
+    ("spi_fslice_normal_ws", ctypes.c_int,
+     [_vp, _vp, ctypes.c_double, _vp, ctypes.c_int, _vp, ctypes.c_longlong, _vp]),
     ("spi_fslice_adjoint64", ctypes.c_int, [_vp, _vp, _vp, _vp]),
     ("spi_fslice_forward64", ctypes.c_int, [_vp, _vp, _vp, _vp]),
     ("spi_fslice_volume", ctypes.c_int, [_vp, _vp, _vp, _vp]),

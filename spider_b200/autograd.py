@@ -105,11 +105,12 @@ class FourierSlicePlan:
     angle list: ``forward`` extracts central slices from a Fourier grid (the
     exact adjoint of ONELINE's insertion, oneline.f:38-200, without the weight
     grid), ``adjoint`` inserts slices into a grid (that insertion), ``normal``
-    applies E^T E + lam I in one fused pass.  Grids are float32 tensors
+    applies E^T E + lam I through a slice buffer.  Grids are float32 tensors
     [2nx, 2nx, nx+1, 2] (complex as (re, im) pairs), slices [nang, 2nx, nx+1, 2]
     in the layout and sign of the staged image spectra (``stage``).  forward,
     adjoint and normal run on torch's current stream, allocate nothing in the
-    library and do not synchronise, so they can be captured in a CUDA graph."""
+    library (normal's buffer comes from torch's allocator) and do not
+    synchronise, so they can be captured in a CUDA graph."""
 
     def __init__(self, nx: int, angles, ctx: ops.Context | None = None, device: int = 0):
         import ctypes
@@ -161,20 +162,30 @@ class FourierSlicePlan:
     def normal(self, grid: torch.Tensor, lam: float, out: torch.Tensor | None = None) -> torch.Tensor:
         if out is None:
             out = torch.empty(self.shape, dtype=torch.float32, device=self.device)
-        ops.check(self._L.spi_fslice_normal(self._h, self._p(grid), float(lam), self._p(out), self._stream()))
+        self._p(grid), self._p(out)
+        return self._normal(grid, lam, out)
+
+    def _normal(self, grid, lam, out):
+        """E^T (E grid) + lam grid through a slice buffer from torch's allocator: one per
+        call, on the call's stream, so calls on several streams do not share it."""
+        import ctypes
+        fp64 = int(grid.dtype == torch.float64)
+        nb = ctypes.c_longlong()
+        ops.check(self._L.spi_fslice_normal_ws_bytes(self._h, fp64, ctypes.byref(nb)))
+        ws = torch.empty(nb.value, dtype=torch.uint8, device=self.device)
+        ops.check(self._L.spi_fslice_normal_ws(self._h, ctypes.c_void_p(grid.data_ptr()), float(lam),
+                                               ctypes.c_void_p(out.data_ptr()), fp64, ctypes.c_void_p(ws.data_ptr()),
+                                               nb.value, self._stream()))
         return out
 
     def normal64(self, grid: torch.Tensor, lam: float, out: torch.Tensor | None = None) -> torch.Tensor:
-        """E^T E + lam I on FP64 grids: FP64 sums and scatter, FP32 table weights."""
-        import ctypes
+        """E^T E + lam I on FP64 grids: FP64 slices and sums, FP32 table weights."""
         if out is None:
             out = torch.empty(self.shape, dtype=torch.float64, device=self.device)
         for t in (grid, out):
             if not (t.is_cuda and t.dtype == torch.float64 and t.is_contiguous()):
                 raise ops.SpiderError(101, "normal64 needs contiguous float64 CUDA tensors")
-        ops.check(self._L.spi_fslice_normal64(self._h, ctypes.c_void_p(grid.data_ptr()), float(lam),
-                                              ctypes.c_void_p(out.data_ptr()), self._stream()))
-        return out
+        return self._normal(grid, lam, out)
 
     def forward64(self, grid: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         """E on an FP64 grid into FP64 slices (FP64 sums of the same taps)."""
@@ -243,7 +254,7 @@ def fourier_slice(grid: torch.Tensor, plan: FourierSlicePlan) -> torch.Tensor:
 class NormalCG:
     """Conjugate gradients on (A^T A + lam I) x = rhs, in fixed device
     buffers; A is the plan's operator (PJ 3Q with PJ3QPlan, the FourierSlice
-    extraction with FourierSlicePlan, whose E^T E + lam I is one fused pass).
+    extraction with FourierSlicePlan, whose normal operator is one call).
     With ``graph`` one iteration is captured once as a CUDA graph and
     replayed.  Dot products and step lengths are FP64; with ``fp64_vectors``
     (the default for the FourierSlice pair, whose eigenvalues spread over

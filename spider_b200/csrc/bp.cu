@@ -21,15 +21,9 @@
 
 #include "../../include/spider_b200.h"
 #include "ctx.h"
+#include "slab.cuh"   // SliceDesc, insert_x4_kernel
 
 namespace spi {
-
-struct SliceDesc {
-  float dm[6];  // DMS(1:6): first two columns of the (symmetrised) rotation
-  int img;      // image index inside the chunk
-  int grid;     // target grid (BP 32F half set)
-};
-static_assert(sizeof(SliceDesc) == 32, "slice descriptor is 32 bytes");
 
 // ----------------------------------------------------------------------------
 // helpers
@@ -1069,21 +1063,6 @@ __global__ void __launch_bounds__(512) insert_xlane_kernel(const void* __restric
 }
 
 // ----------------------------------------------------------------------------
-// G[i] += v as one 16-byte reduction in L2 (red.global.add.v4.f32).  The
-// address is converted to the global window explicitly: insert_x4_kernel
-// takes its grid pointer from shared memory, and on such a generic pointer
-// atomicAdd(float4*) was not compiled to the vector reduction
-// (measured: 1.9x the instructions and no L2 reduction requests; 205
-// against 156 ms for the same 10,000 images at 256^3).
-__device__ __forceinline__ void red_add_v4(float4* p, float4 v) {
-  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "f"(v.x),
-               "f"(v.y), "f"(v.z), "f"(v.w));
-}
-
-}  // namespace spi
-#include "slab.cuh"   // insert_x4_kernel
-namespace spi {
-
 // True when the table is zero from distance 1.805 on, as FILLBESSIL's are
 // (0.9 of the two-voxel half width): at most four consecutive taps of the five
 // are then nonzero and columns within kSlabR of a pixel hold them all
@@ -2227,24 +2206,6 @@ static SlabClass slab_class(const spi_ctx* c, const void* spec, const SliceDesc*
   return m;
 }
 
-// Work items of the classes: a slice's row of tiles each, or its parts when
-// all rows together would give the launch's CTAs fewer than eight items (the
-// tail of a launch is about half an item per CTA: 200 slices at 64^3 0.148
-// against 0.176 ms with whole rows).  Returns their number.
-static long long slab_items(int sm_count, SlabClass* cls, int ncls) {
-  auto rows_of = [](const SlabClass& m) { return (long long)m.nslices * ((2 * m.nx + kSlabTile - 1) / kSlabTile); };
-  long long rows = 0, items = 0;
-  for (int k = 0; k < ncls; ++k) rows += rows_of(cls[k]);
-  const long long want = 8LL * kSlabBlocks * sm_count;
-  for (int k = 0; k < ncls; ++k) {
-    const long long most = (cls[k].nx + kSlabTile - 1) / kSlabTile;
-    cls[k].parts = (int)std::max(1LL, std::min(most, rows > 0 ? (want + rows - 1) / rows : 1LL));
-    cls[k].item0 = items;
-    items += rows_of(cls[k]) * cls[k].parts;
-  }
-  return items;
-}
-
 // insert_x4_kernel over the items of a, persistent; `work` is zeroed first
 static int launch_slab(spi_ctx* c, const SlabArgs& a, bool bf16, unsigned long long* work, int per_sm, cudaStream_t st) {
   SPI_CUDA(cudaMemsetAsync(work, 0, sizeof(unsigned long long), st));
@@ -2259,8 +2220,8 @@ static int launch_slab(spi_ctx* c, const SlabArgs& a, bool bf16, unsigned long l
     kern<<<insert_blocks(c, kern, kSlabThreads + 32, smem, per_sm), kSlabThreads + 32, smem, st>>>(a, work);
     return check_kernel("insert_x4_kernel");
   };
-  if (bf16) return go(insert_x4_kernel<true>, sizeof(SlabSmem<true>));
-  return go(insert_x4_kernel<false>, sizeof(SlabSmem<false>));
+  if (bf16) return go(insert_x4_kernel<SlabBpBf16>, sizeof(SlabSmem<SlabBpBf16>));
+  return go(insert_x4_kernel<SlabBp>, sizeof(SlabSmem<SlabBp>));
 }
 
 static int launch_insert(spi_ctx* c, const SliceDesc* sl, int nslices, float4* g1) {
@@ -2285,7 +2246,7 @@ static int launch_insert(spi_ctx* c, const SliceDesc* sl, int nslices, float4* g
       SlabArgs a{};
       a.ncls = 1;
       a.cls[0] = slab_class(c, spec, sl, nslices, g0, g1);
-      a.nitems = slab_items(c->sm_count, a.cls, 1);
+      a.nitems = slab_items((long long)kSlabBlocks * c->sm_count, a.cls, 1);
       SPI_TRY(c->workctr.ensure(sizeof(unsigned long long)));
       SPI_TRY(launch_slab(c, a, c->bf16, c->workctr.as<unsigned long long>(), c->insert_blocks_per_sm, c->stream));
     } else {
@@ -2756,7 +2717,7 @@ static int bp_insert_multi_impl(spi_ctx* const* ctxs, int ncls, const float* con
     if (nc == 0) continue;
     SPI_CUDA(cudaStreamWaitEvent(st, lead->ev_ready[h], 0));
     args.ncls = nc;
-    args.nitems = slab_items(lead->sm_count, args.cls, nc);
+    args.nitems = slab_items((long long)kSlabBlocks * lead->sm_count, args.cls, nc);
     int ev = lead->phase_begin(2, st);
     SPI_TRY(launch_slab(lead, args, lead->bf16, lead->workctr.as<unsigned long long>(), env_int("SPI_MC_BLOCKS_PER_SM", kSlabBlocks), st));
     lead->phase_end(ev);

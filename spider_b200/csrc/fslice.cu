@@ -9,17 +9,20 @@
 //       adjoint of the insertion below;
 //   E^T (adjoint, insertion):   slices T -> grid X, ONELINE's X += BTQ * W
 //       with the weight grid dropped;
-//   E^T E + lam I (normal):     one fused pass that gathers each pixel's taps
-//       and scatters the sum back over the same taps.
+//   E^T E + lam I (normal):     E into a slice buffer and E^T of it, or,
+//       without a buffer, one pass that gathers each pixel's taps and
+//       scatters the sum back over the same taps.
 //
 // Grid: complex float2 [2nx][2nx][nx+1] (i fastest, Fortran X(0:NX,N,N)).
 // Slices: float2 [nslice][2nx][nx+1] in the layout and sign of the staged
 // spectra the back-projection inserts (cuFFT R2C of the padded, shifted
 // image; ONELINE's BI is its conjugate).  Every tap -- voxel, table weight,
 // Hermitian flip (x < 0), reflected point (oneline.f:118-150) -- is computed
-// exactly as insert_x4_kernel computes it, four lanes per pixel over the
-// nonzero window of the table.
+// that of the back-projection's insertion: E is fs_extract.cuh, E^T the column
+// insertion of slab.cuh; the normal operators without a buffer take four lanes
+// per pixel over the nonzero window of the table.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -27,15 +30,10 @@
 
 #include "../../include/spider_b200.h"
 #include "ctx.h"
+#include "fs_extract.cuh"
+#include "slab.cuh"
 
 namespace spi {
-
-struct FsDesc {
-  float dm[6];  // DM(1:6) of the slice (CANG, cang.f:44-81)
-  int img;      // slice index
-  int cols;     // order of the insertion and normal kernels: 0 row by row, 1 by half columns
-};
-static_assert(sizeof(FsDesc) == 32, "slice descriptor is 32 bytes");
 
 __device__ __forceinline__ int fs_nint_pos(float v) {  // Fortran NINT, v >= 0
   const float f = floorf(v);
@@ -43,44 +41,6 @@ __device__ __forceinline__ int fs_nint_pos(float v) {  // Fortran NINT, v >= 0
 }
 __device__ __forceinline__ float fs_tap(const float* tab, float v, int k, float fltb) {
   return tab[fs_nint_pos(__fmul_rn(fabsf(__fsub_rn(v, (float)k)), fltb))];
-}
-
-// Line r (0 <= r < N) of a slice: row J = r - NX + 1 (pixels consecutive in
-// I) or, for a slice marked cols, half of column I = r / 2 (pixels
-// consecutive in J; J >= 0 for even r, J < 0 for odd r).  Pixel k of the line
-// is (i0 + di k, j0 + dj k), k < cnt: the pixels of the line inside the half
-// disc of oneline.f's loops, so every pixel of the slice lies on exactly one
-// line in either order.  The host marks slices as the back-projection does
-// (bp.cu, insert_line_x4): eight pixels stepping along z scatter into eight
-// grid planes 2 MB apart at 256^3.  Only the insertions E^T follow the mark
-// (use_cols): at 256^3 with 8,192 slices it took E^T from 158.6 to 111.7 ms,
-// while the fused normal operators, which gather before they scatter, were
-// 2% slower with it (0.363 against 0.356 s per CG iteration in FP64).
-struct FsLine {
-  int i0, j0, di, dj, cnt;
-};
-__device__ __forceinline__ int fs_isqrt_below(int rem) {   // the largest m >= 0 with m * m < rem (rem > 0)
-  // approximate square root (no IEEE slow path); the two loops make m exact
-  float f;
-  asm("sqrt.approx.f32 %0, %1;" : "=f"(f) : "f"((float)(rem - 1)));
-  int m = (int)f;
-  while (m > 0 && m * m >= rem) --m;
-  while ((m + 1) * (m + 1) < rem) ++m;
-  return m;
-}
-__device__ __forceinline__ FsLine fs_line(const FsDesc& sd, int r, int nx, bool use_cols) {
-  const int NN4 = nx * nx;
-  FsLine l;
-  if (!(use_cols && sd.cols)) {
-    l.j0 = r - nx + 1; l.i0 = 0; l.di = 1; l.dj = 0;
-    l.cnt = (l.j0 * l.j0 < NN4) ? fs_isqrt_below(NN4 - l.j0 * l.j0) + 1 : 0;
-  } else {
-    l.i0 = r >> 1; l.di = 0;
-    const int jm = fs_isqrt_below(NN4 - l.i0 * l.i0);
-    if (r & 1) { l.j0 = -1; l.dj = -1; l.cnt = l.i0 == 0 ? 0 : jm; }
-    else { l.j0 = 0; l.dj = 1; l.cnt = jm + 1; }
-  }
-  return l;
 }
 
 // The tap window of pixel (I, J) for lane q of its four-lane group (lanes
@@ -94,10 +54,7 @@ struct FsWin {
   float ty[4], tz[4];
 };
 
-// LS: lanes per x tap in the pixel's lane group (the y/z weight of window
-// position l lives in lane gl + l * LS).
-template <int LS = 1>
-__device__ __forceinline__ void fs_window(const FsDesc& sd, int I, int J, int nx, const float* tab, float fltb,
+__device__ __forceinline__ void fs_window(const SliceDesc& sd, int I, int J, int nx, const float* tab, float fltb,
                                           int q, int gl, FsWin& w) {
   const int N = 2 * nx, N2 = nx, LN2 = 2, NN4 = N * N / 4;
   const float fN = (float)N;
@@ -125,8 +82,8 @@ __device__ __forceinline__ void fs_window(const FsDesc& sd, int I, int J, int nx
   const float tzq = fs_tap(tab, znew, w.zs + q, fltb);
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    w.ty[l] = __shfl_sync(0xffffffffu, tyq, gl + l * LS);
-    w.tz[l] = __shfl_sync(0xffffffffu, tzq, gl + l * LS);
+    w.ty[l] = __shfl_sync(0xffffffffu, tyq, gl + l);
+    w.tz[l] = __shfl_sync(0xffffffffu, tzq, gl + l);
   }
   w.ok = ok && w.tx != 0.0f;
 }
@@ -198,69 +155,31 @@ __device__ __forceinline__ float2 group_sum4(float2 v) {   // sum over the four 
   return v;
 }
 
-// MODE 0: extraction E (X -> T), 1: insertion E^T (T -> X), 2: normal E^T E
-// (P -> Q, Q pre-set to lam * P).  A warp takes one row J of one slice
-// (rows handed out in slice-major order by a grid stride), eight pixels at a
-// time.
-template <int MODE>
-__global__ void __launch_bounds__(256) fs_kernel(const float2* __restrict__ in, float2* __restrict__ out,
-                                                 const FsDesc* __restrict__ slices, int nslices, int nx,
-                                                 const float* __restrict__ kbtab, float fltb) {
+// The normal operator E^T E without a slice buffer (P -> Q, Q pre-set to lam *
+// P), for callers that give none: a warp takes one row J of one slice (rows
+// handed out in slice-major order by a grid stride), eight pixels at a time,
+// gathers each pixel's taps and scatters the sum back over them.
+__global__ void __launch_bounds__(256) fs_normal_kernel(const float2* __restrict__ in, float2* __restrict__ out,
+                                                        const SliceDesc* __restrict__ slices, int nslices, int nx,
+                                                        const float* __restrict__ kbtab, float fltb) {
   extern __shared__ float tab[];
   for (int i = threadIdx.x; i < 5000; i += blockDim.x) tab[i] = kbtab[i];
   __syncthreads();
-  const int N = 2 * nx, NN4 = N * N / 4;
+  const int N = 2 * nx, NN4 = nx * nx;
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2, q = lane & 3, gl = lane & ~3;
   const long long nitems = (long long)nslices * N;
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  const size_t rowlen = (size_t)(nx + 1);
-  const size_t plane = (size_t)N * rowlen;
   for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < nitems;
        item += warps) {
-    const int s = (int)(item / N);
-    const FsDesc sd = slices[s];
-    if (MODE == 0) {
-      // rows only: every pixel of the row is written, zero outside the disc
-      const int J = (int)(item % N) - nx + 1;
-      const int JP = (J >= 0) ? J : N + J;
-      const size_t srow = (size_t)sd.img * plane + (size_t)JP * rowlen;
-      int I0 = 0;
-      for (; I0 <= nx && I0 * I0 + J * J < NN4; I0 += 8) {   // warp-uniform
-        const int I = I0 + g;
-        FsWin w;
-        fs_window(sd, I, J, nx, tab, fltb, q, gl, w);
-        const float2 acc = group_sum4(fs_gather(in, w, q, nx));
-        // BI_adj = acc (conj'ed for a flipped pixel); T = conj(BI_adj)
-        if (q == 0 && I <= nx) {
-          float2 t = make_float2(0.0f, 0.0f);
-          if (I * I + J * J < NN4 && !(I == 0 && J < 0)) t = w.flipped ? acc : make_float2(acc.x, -acc.y);
-          out[srow + I] = t;
-        }
-      }
-      for (int I = I0 + lane; I <= nx; I += 32) out[srow + I] = make_float2(0.0f, 0.0f);
-    } else {
-      const FsLine ln = fs_line(sd, (int)(item % N), nx, MODE == 1);
-      for (int k0 = 0; k0 < ln.cnt; k0 += 8) {   // warp-uniform
-        const int k = k0 + g;
-        const int I = ln.i0 + ln.di * k, J = ln.j0 + ln.dj * k;
-        FsWin w;
-        fs_window(sd, I, J, nx, tab, fltb, q, gl, w);
-        if (MODE == 1) {
-          // BTQ = BI = conj(T), or conj(BI) = T for a flipped pixel
-          float2 b = make_float2(0.0f, 0.0f);
-          if (w.ok) {
-            const int JP = (J >= 0) ? J : N + J;
-            const float2 t = in[(size_t)sd.img * plane + (size_t)JP * rowlen + I];
-            b = w.flipped ? t : make_float2(t.x, -t.y);
-          }
-          fs_scatter(out, w, q, nx, b);
-        } else {
-          // extraction then insertion of the same pixel: the flips cancel
-          const float2 sum = group_sum4(fs_gather(in, w, q, nx));
-          fs_scatter(out, w, q, nx, sum);
-        }
-      }
+    const SliceDesc sd = slices[item / N];
+    const int J = (int)(item % N) - nx + 1;
+    for (int I0 = 0; I0 * I0 + J * J < NN4; I0 += 8) {   // warp-uniform
+      FsWin w;
+      fs_window(sd, I0 + g, J, nx, tab, fltb, q, gl, w);
+      // extraction then insertion of the same pixel: the flips cancel
+      const float2 sum = group_sum4(fs_gather(in, w, q, nx));
+      fs_scatter(out, w, q, nx, sum);
     }
   }
 }
@@ -269,58 +188,12 @@ __global__ void __launch_bounds__(256) fs_kernel(const float2* __restrict__ in, 
 // grids, the pixel sums and the scatter (FP64 atomics) in double precision.
 // Late CG iterations apply E^T E to directions whose image is much smaller
 // than ||E^T E|| ||p||; FP32 sums would lose that many digits there.
-__device__ __forceinline__ double2 fs_gather64(const double2* __restrict__ X, const FsWin& w, int q, int nx) {
-  double2 acc = make_double2(0.0, 0.0);
-  if (!w.ok) return acc;
-#pragma unroll
-  for (int lz = 0; lz < 4; ++lz) {
-    if (w.tz[lz] == 0.0f) continue;
-#pragma unroll
-    for (int ly = 0; ly < 4; ++ly) {
-      const float tyz = __fmul_rn(w.ty[ly], w.tz[lz]);
-      if (tyz == 0.0f) continue;
-      const float wg = __fmul_rn(w.tx, tyz);
-      if (wg == 0.0f) continue;
-      bool refl;
-      const double2 v = X[fs_voxel(w, q, ly, lz, nx, refl)];
-      const double d = (double)wg;
-      acc.x = __dadd_rn(acc.x, __dmul_rn(v.x, d));
-      acc.y = refl ? __dsub_rn(acc.y, __dmul_rn(v.y, d)) : __dadd_rn(acc.y, __dmul_rn(v.y, d));
-    }
-  }
-  return acc;
-}
-
-__device__ __forceinline__ void fs_scatter64(double2* __restrict__ X, const FsWin& w, int q, int nx, double2 b) {
-  if (!w.ok) return;
-#pragma unroll
-  for (int lz = 0; lz < 4; ++lz) {
-    if (w.tz[lz] == 0.0f) continue;
-#pragma unroll
-    for (int ly = 0; ly < 4; ++ly) {
-      const float tyz = __fmul_rn(w.ty[ly], w.tz[lz]);
-      if (tyz == 0.0f) continue;
-      const float wg = __fmul_rn(w.tx, tyz);
-      if (wg == 0.0f) continue;
-      bool refl;
-      double* v = reinterpret_cast<double*>(X + fs_voxel(w, q, ly, lz, nx, refl));
-      const double d = (double)wg;
-      atomicAdd(v, __dmul_rn(b.x, d));
-      atomicAdd(v + 1, refl ? -__dmul_rn(b.y, d) : __dmul_rn(b.y, d));
-    }
-  }
-}
-
-// NORMAL: E^T E of an FP64 grid; else E^T of FP32 slices (`sl_in`) into an
-// FP64 grid.
-// In the normal operator the lane's 16 voxel offsets come from four plane and
+// The lane's 16 voxel offsets come from four plane and
 // four row terms computed once per pixel (32-bit: a grid has < 2^32 voxels up
 // to nx = 512) and serve both the gather and the scatter (measured 2-3%
 // faster than computing each tap's index twice, 48 instead of 57 registers).
-template <bool NORMAL>
-__global__ void __launch_bounds__(256) fs_normal64_kernel(const double2* __restrict__ in, const float2* __restrict__ sl_in,
-                                                          double2* __restrict__ out,
-                                                          const FsDesc* __restrict__ slices, int nslices, int nx,
+__global__ void __launch_bounds__(256) fs_normal64_kernel(const double2* __restrict__ in, double2* __restrict__ out,
+                                                          const SliceDesc* __restrict__ slices, int nslices, int nx,
                                                           const float* __restrict__ kbtab, float fltb) {
   extern __shared__ float tab[];
   for (int i = threadIdx.x; i < 5000; i += blockDim.x) tab[i] = kbtab[i];
@@ -332,16 +205,13 @@ __global__ void __launch_bounds__(256) fs_normal64_kernel(const double2* __restr
   const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
   for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < nitems;
        item += warps) {
-    const int s = (int)(item / N);
-    const FsDesc sd = slices[s];
-    const FsLine ln = fs_line(sd, (int)(item % N), nx, !NORMAL);
-    for (int k0 = 0; k0 < ln.cnt; k0 += 8) {   // warp-uniform
-      const int k = k0 + g;
-      const int I = ln.i0 + ln.di * k, J = ln.j0 + ln.dj * k;
+    const SliceDesc sd = slices[item / N];
+    const int J = (int)(item % N) - nx + 1;
+    for (int I0 = 0; I0 * I0 + J * J < nx * nx; I0 += 8) {   // warp-uniform
       FsWin w;
-      fs_window(sd, I, J, nx, tab, fltb, q, gl, w);
+      fs_window(sd, I0 + g, J, nx, tab, fltb, q, gl, w);
       double2 v;
-      if (NORMAL) {
+      {
         const int ixp = w.xs + q;
         const bool refl = ixp < 0;
         const unsigned ixa = (unsigned)(refl ? -ixp : ixp);
@@ -392,116 +262,19 @@ __global__ void __launch_bounds__(256) fs_normal64_kernel(const double2* __restr
             atomicAdd(o + 1, refl ? -__dmul_rn(v.y, d) : __dmul_rn(v.y, d));
           }
         }
-        continue;
-      } else {   // BTQ = BI = conj(T), or T for a flipped pixel
-        v = make_double2(0.0, 0.0);
-        if (w.ok) {
-          const int JP = (J >= 0) ? J : N + J;
-          const float2 t = sl_in[((size_t)sd.img * N + JP) * (size_t)(nx + 1) + I];
-          v = make_double2((double)t.x, w.flipped ? (double)t.y : -(double)t.y);
-        }
-      }
-      fs_scatter64(out, w, q, nx, v);
-    }
-  }
-}
-
-// E^T into an FP64 grid with eight lanes per pixel: lane 8g + 2q + h takes x
-// tap q of pixel g and the real (h = 0) or imaginary (h = 1) part.  There is
-// no 16-byte FP64 reduction, so in the four-lane form every tap's complex add
-// is two 8-byte reductions from one lane, the real parts of a pixel's four
-// taps (16 bytes apart) in one instruction and the imaginary parts in
-// another; here one instruction adds both parts of four consecutive voxels
-// (64 contiguous bytes), half the L2 reduction requests and sectors.
-// Measured with 10,000 and 8,192 slices: 71.8 against 84.0 ms at 128^3,
-// 239 against 291 ms at 256^3.  The fused normal operator keeps four lanes: its
-// gather, with every weight and voxel index computed by two lanes here, made
-// it 1.7x slower in this form (0.159 against 0.0945 s per CG iteration), and
-// a four-lane gather followed by this scatter in two passes (the windows and
-// pixel sums moved across lanes by shuffles) 1.3x slower (0.123 s).
-__global__ void __launch_bounds__(256) fs_insert64w_kernel(const float2* __restrict__ sl_in, double* __restrict__ out,
-                                                           const FsDesc* __restrict__ slices, int nslices, int nx,
-                                                           const float* __restrict__ kbtab, float fltb) {
-  extern __shared__ float tab[];
-  for (int i = threadIdx.x; i < 5000; i += blockDim.x) tab[i] = kbtab[i];
-  __syncthreads();
-  const int N = 2 * nx;
-  const int lane = threadIdx.x & 31;
-  const int g = lane >> 3, q = (lane >> 1) & 3, h = lane & 1, gl = lane & ~7;
-  const long long nitems = (long long)nslices * N;
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < nitems;
-       item += warps) {
-    const int s = (int)(item / N);
-    const FsDesc sd = slices[s];
-    const FsLine ln = fs_line(sd, (int)(item % N), nx, true);
-    for (int k0 = 0; k0 < ln.cnt; k0 += 4) {   // warp-uniform
-      const int k = k0 + g;
-      const int I = ln.i0 + ln.di * k, J = ln.j0 + ln.dj * k;
-      FsWin w;
-      fs_window<2>(sd, I, J, nx, tab, fltb, q, gl, w);
-      if (!w.ok) continue;
-      // BTQ = BI = conj(T), or T for a flipped pixel
-      const int JP = (J >= 0) ? J : N + J;
-      const float2 t = sl_in[((size_t)sd.img * N + JP) * (size_t)(nx + 1) + I];
-      const double v = h ? (w.flipped ? (double)t.y : -(double)t.y) : (double)t.x;
-#pragma unroll
-      for (int lz = 0; lz < 4; ++lz) {
-        if (w.tz[lz] == 0.0f) continue;
-#pragma unroll
-        for (int ly = 0; ly < 4; ++ly) {
-          const float tyz = __fmul_rn(w.ty[ly], w.tz[lz]);
-          if (tyz == 0.0f) continue;
-          const float wg = __fmul_rn(w.tx, tyz);
-          if (wg == 0.0f) continue;
-          bool refl;
-          const size_t vx = fs_voxel(w, q, ly, lz, nx, refl);
-          const double tw = __dmul_rn(v, (double)wg);
-          atomicAdd(out + 2 * vx + h, (h && refl) ? -tw : tw);
-        }
       }
     }
   }
 }
 
-// Extraction E on an FP64 grid into FP64 slices (FP64 sums of the same taps):
-// an exact reference of the FP32 extraction for gradient checks.
-__global__ void __launch_bounds__(256) fs_extract64_kernel(const double2* __restrict__ in, double2* __restrict__ out,
-                                                           const FsDesc* __restrict__ slices, int nslices, int nx,
-                                                           const float* __restrict__ kbtab, float fltb) {
-  extern __shared__ float tab[];
-  for (int i = threadIdx.x; i < 5000; i += blockDim.x) tab[i] = kbtab[i];
-  __syncthreads();
-  const int N = 2 * nx, NN4 = N * N / 4;
-  const int lane = threadIdx.x & 31;
-  const int g = lane >> 2, q = lane & 3, gl = lane & ~3;
-  const long long nitems = (long long)nslices * N;
-  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < nitems;
-       item += warps) {
-    const int s = (int)(item / N);
-    const int J = (int)(item % N) - nx + 1;
-    const FsDesc sd = slices[s];
-    const int JP = (J >= 0) ? J : N + J;
-    const size_t srow = ((size_t)sd.img * N + JP) * (size_t)(nx + 1);
-    int I0 = 0;
-    for (; I0 <= nx && I0 * I0 + J * J < NN4; I0 += 8) {   // warp-uniform
-      const int I = I0 + g;
-      FsWin w;
-      fs_window(sd, I, J, nx, tab, fltb, q, gl, w);
-      double2 v = fs_gather64(in, w, q, nx);
-      v.x = __dadd_rn(v.x, __shfl_xor_sync(0xffffffffu, v.x, 1));
-      v.y = __dadd_rn(v.y, __shfl_xor_sync(0xffffffffu, v.y, 1));
-      v.x = __dadd_rn(v.x, __shfl_xor_sync(0xffffffffu, v.x, 2));
-      v.y = __dadd_rn(v.y, __shfl_xor_sync(0xffffffffu, v.y, 2));
-      if (q == 0 && I <= nx) {
-        double2 t = make_double2(0.0, 0.0);
-        if (I * I + J * J < NN4 && !(I == 0 && J < 0)) t = w.flipped ? v : make_double2(v.x, -v.y);
-        out[srow + I] = t;
-      }
-    }
-    for (int I = I0 + lane; I <= nx; I += 32) out[srow + I] = make_double2(0.0, 0.0);
-  }
+// E^T: the column insertion into complex grids (slab.cuh).  us per slice, with
+// per-tap reductions -> now: FP32 128^3 2.96 -> 2.03, 256^3 12.1 -> 7.75; FP64
+// 7.26 -> 3.33 and 29.4 -> 12.6.  The FP64 normal operator (E and E^T through
+// the buffer): 9.50 -> 6.40 and 43.8 -> 27.0; FP32 6.56 -> 4.2 and 34.6 -> 17.3.
+template <class F>
+__global__ void __launch_bounds__(kSlabThreads + 32, F::D ? kSlabBlocks64 : kSlabBlocks)
+    fs_insert_kernel(const __grid_constant__ SlabArgs P, unsigned long long* __restrict__ work) {
+  slab_main<F>(P, work);
 }
 
 __global__ void fs_scale64_kernel(const double2* __restrict__ p, double lam, double2* __restrict__ q, size_t n) {
@@ -571,7 +344,7 @@ using namespace spi;
 struct spi_fslice_plan {
   spi_ctx* ctx = nullptr;
   int device = 0, nx = 0, n = 0, nang = 0, sm_count = 148;
-  FsDesc* sl = nullptr;        // [nang]
+  SliceDesc* sl = nullptr;        // [nang]
   float* tab = nullptr;        // KB table, 5000 floats
   float fltb = 0.0f;
   float* wkb = nullptr;        // |WKB(LR)|, LR = 0..(nx/2)^2
@@ -586,17 +359,84 @@ struct spi_fslice_plan {
 namespace {
 
 int fs_blocks(const spi_fslice_plan* p) { return p->sm_count * 3; }
-// E^T into FP64 with eight lanes per pixel (SPI_FS_LANES=4 selects the four-lane form)
-bool fs_w8() {
-  const char* e = std::getenv("SPI_FS_LANES");
-  return !(e && std::atoi(e) == 4);
-}
 int fs_grid_blocks(const spi_fslice_plan* p, size_t work) {
   size_t b = (work + 255) / 256, cap = (size_t)p->sm_count * 8;
   return (int)std::max<size_t>(1, std::min(b, cap));
 }
 size_t fs_grid_elems(const spi_fslice_plan* p) { return (size_t)(p->nx + 1) * p->n * p->n; }
 constexpr size_t kFsSmem = 5000 * sizeof(float);
+// work counters of the normal operator's insertion launches, `chunk` slices each
+long long fs_counter_bytes(const spi_fslice_plan* p, long long chunk) {
+  return (p->nang + chunk - 1) / chunk * (long long)sizeof(unsigned long long);
+}
+size_t fs_plane(const spi_fslice_plan* p) { return (size_t)p->n * (p->nx + 1); }
+
+// per-device attributes of the extraction and insertion kernels
+int fs_set_attributes(int device) {
+  static std::atomic<unsigned long long> done{0};
+  const unsigned long long bit = 1ull << (device & 63);
+  if (done.load() & bit) return 0;
+  auto set = [](auto kern, size_t smem) {
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  };
+  SPI_CUDA(set(fs_insert_kernel<SlabFs>, sizeof(SlabSmem<SlabFs>)));
+  SPI_CUDA(set(fs_insert_kernel<SlabFs64>, sizeof(SlabSmem<SlabFs64>)));
+  SPI_CUDA(set(fs_insert_kernel<SlabFs64d>, sizeof(SlabSmem<SlabFs64d>)));
+  done.fetch_or(bit);
+  return 0;
+}
+
+template <class F>
+int fs_insert(const spi_fslice_plan* p, const void* slices, void* grid, int first, int count, unsigned long long* work,
+              cudaStream_t s);
+
+// grid = E^T of all slices.  The work counter of the launch is a voxel of the
+// output that no tap reaches, (x, y, z) = (NX, 0, 0): the plan may run on
+// several streams at once, so the counter has to be the call's own.
+template <class F>
+int fs_adjoint(const spi_fslice_plan* p, const void* slices, void* grid, size_t voxel, cudaStream_t s) {
+  SPI_CUDA(cudaMemsetAsync(grid, 0, fs_grid_elems(p) * voxel, s));
+  auto* work = reinterpret_cast<unsigned long long*>(static_cast<char*>(grid) + (size_t)p->nx * voxel);
+  SPI_TRY(fs_insert<F>(p, slices, grid, 0, p->nang, work, s));
+  SPI_CUDA(cudaMemsetAsync(work, 0, sizeof(*work), s));
+  return 0;
+}
+
+// E of slices [first, first + count) of the plan into out (its first slice first)
+template <class T2>
+int fs_extract(const spi_fslice_plan* p, const void* grid, void* out, int first, int count, cudaStream_t s) {
+  const long long rows = ((long long)count * p->n + kExThreads / 32 - 1) / (kExThreads / 32);
+  const int blocks = (int)std::min<long long>(rows, (long long)p->sm_count * ExBlocks<T2>::value);
+  fs_extract_kernel<T2><<<blocks, kExThreads, 0, s>>>(static_cast<const T2*>(grid), static_cast<T2*>(out), p->sl + first,
+                                                      count, p->nx, p->tab, p->fltb);
+  SPI_TRY(check_kernel("fs_extract_kernel"));
+  p->ctx->count();
+  return 0;
+}
+
+// grid += E^T of slices [first, first + count), whose values start at
+// `slices`; *work (device) is zero
+template <class F>
+int fs_insert(const spi_fslice_plan* p, const void* slices, void* grid, int first, int count, unsigned long long* work,
+              cudaStream_t s) {
+  SlabArgs a{};
+  a.ncls = 1;
+  SlabClass& m = a.cls[0];
+  // descriptors hold the slices' indices in the plan
+  m.spec = static_cast<const typename F::Raw*>(slices) - (ptrdiff_t)first * (ptrdiff_t)fs_plane(p);
+  m.slices = p->sl + first;
+  m.g0 = m.g1 = grid;
+  m.tab = p->tab;
+  m.nx = p->nx;
+  m.nslices = count;
+  m.fltb = p->fltb;
+  const long long most = (long long)p->sm_count * (F::D ? kSlabBlocks64 : kSlabBlocks);
+  a.nitems = slab_items(most, a.cls, 1);
+  fs_insert_kernel<F><<<(int)std::min(most, a.nitems), kSlabThreads + 32, sizeof(SlabSmem<F>), s>>>(a, work);
+  SPI_TRY(check_kernel("fs_insert_kernel"));
+  p->ctx->count();
+  return 0;
+}
 
 }  // namespace
 
@@ -611,23 +451,21 @@ int spi_fslice_plan_create(spi_ctx* ctx, int nx, const float* angles, int nang, 
   KBTab kb;
   fill_kb(2 * nx, kb);
   {
-    const int i0 = std::max(0, (int)std::floor(2.0 * kb.fltb) - 1);
+    // zero from distance 1.805 on, as FILLBESSIL's tables are
+    const int i0 = std::max(0, (int)std::floor(1.805 * kb.fltb));
     for (int i = i0; i < 5000; ++i)
       if (kb.tab[i] != 0.0f)
         return fail(kInvalid, "spi_fslice_plan_create: the interpolation table of nx = %d has more than four "
                               "nonzero taps per axis", nx);
   }
-  std::vector<FsDesc> hs(nang);
-  const char* ord = std::getenv("SPI_INSERT_ORDER");
-  const int order = !ord ? 1 : std::strcmp(ord, "rows") == 0 ? 0 : std::strcmp(ord, "cols") == 0 ? 2 : 1;
+  SPI_TRY(fs_set_attributes(ctx->device));
+  std::vector<SliceDesc> hs(nang);
   for (int a = 0; a < nang; ++a) {
     float dm[9];
     cang(angles[3 * a + 2], angles[3 * a + 1], angles[3 * a + 0], dm);   // BUILDM1 (bp3f.f:1287)
     std::memcpy(hs[a].dm, dm, 6 * sizeof(float));
     hs[a].img = a;
-    // insertion order (FsLine): the in-plane axis with the smaller z
-    // component, for boxes above 192 (as the back-projection chooses)
-    hs[a].cols = (order == 2 || (order == 1 && nx > 192 && std::fabs(dm[5]) < std::fabs(dm[2]))) ? 1 : 0;
+    hs[a].grid = 0;
   }
   std::vector<float> wkb;
   windkb_table(nx, kb, wkb);
@@ -639,10 +477,10 @@ int spi_fslice_plan_create(spi_ctx* ctx, int nx, const float* angles, int nang, 
   p->n = 2 * nx;
   p->nang = nang;
   p->fltb = kb.fltb;
-  cudaError_t e = cudaMalloc(&p->sl, sizeof(FsDesc) * nang);
+  cudaError_t e = cudaMalloc(&p->sl, sizeof(SliceDesc) * nang);
   if (e == cudaSuccess) e = cudaMalloc(&p->tab, sizeof(kb.tab));
   if (e == cudaSuccess) e = cudaMalloc(&p->wkb, wkb.size() * sizeof(float));
-  if (e == cudaSuccess) e = cudaMemcpy(p->sl, hs.data(), sizeof(FsDesc) * nang, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(p->sl, hs.data(), sizeof(SliceDesc) * nang, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(p->tab, kb.tab, sizeof(kb.tab), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(p->wkb, wkb.data(), wkb.size() * sizeof(float), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
@@ -708,24 +546,13 @@ int spi_fslice_stage(spi_fslice_plan* p, const float* imgs, float* slices, void*
 int spi_fslice_forward(const spi_fslice_plan* p, const float* grid, float* slices, void* stream) {
   if (!p || !grid || !slices) return fail(kInvalid, "spi_fslice_forward: NULL argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  fs_kernel<0><<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const float2*>(grid),
-                                                   reinterpret_cast<float2*>(slices), p->sl, p->nang, p->nx, p->tab,
-                                                   p->fltb);
-  SPI_TRY(check_kernel("fs_kernel<extract>"));
-  p->ctx->count();
-  return 0;
+  return fs_extract<float2>(p, grid, slices, 0, p->nang, s);
 }
 
 int spi_fslice_adjoint(const spi_fslice_plan* p, const float* slices, float* grid, void* stream) {
   if (!p || !grid || !slices) return fail(kInvalid, "spi_fslice_adjoint: NULL argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  SPI_CUDA(cudaMemsetAsync(grid, 0, fs_grid_elems(p) * sizeof(float2), s));
-  fs_kernel<1><<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const float2*>(slices),
-                                                   reinterpret_cast<float2*>(grid), p->sl, p->nang, p->nx, p->tab,
-                                                   p->fltb);
-  SPI_TRY(check_kernel("fs_kernel<insert>"));
-  p->ctx->count();
-  return 0;
+  return fs_adjoint<SlabFs>(p, slices, grid, sizeof(float2), s);
 }
 
 int spi_fslice_normal(const spi_fslice_plan* p, const float* grid_in, float lam, float* grid_out, void* stream) {
@@ -736,10 +563,10 @@ int spi_fslice_normal(const spi_fslice_plan* p, const float* grid_in, float lam,
   fs_scale_kernel<<<fs_grid_blocks(p, ne), 256, 0, s>>>(reinterpret_cast<const float2*>(grid_in), lam,
                                                         reinterpret_cast<float2*>(grid_out), ne);
   SPI_TRY(check_kernel("fs_scale_kernel"));
-  fs_kernel<2><<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const float2*>(grid_in),
+  fs_normal_kernel<<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const float2*>(grid_in),
                                                    reinterpret_cast<float2*>(grid_out), p->sl, p->nang, p->nx, p->tab,
                                                    p->fltb);
-  SPI_TRY(check_kernel("fs_kernel<normal>"));
+  SPI_TRY(check_kernel("fs_normal_kernel"));
   p->ctx->count(2);
   return 0;
 }
@@ -752,9 +579,9 @@ int spi_fslice_normal64(const spi_fslice_plan* p, const double* grid_in, double 
   fs_scale64_kernel<<<fs_grid_blocks(p, ne), 256, 0, s>>>(reinterpret_cast<const double2*>(grid_in), lam,
                                                           reinterpret_cast<double2*>(grid_out), ne);
   SPI_TRY(check_kernel("fs_scale64_kernel"));
-  fs_normal64_kernel<true><<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const double2*>(grid_in), nullptr,
-                                                              reinterpret_cast<double2*>(grid_out), p->sl, p->nang,
-                                                              p->nx, p->tab, p->fltb);
+  fs_normal64_kernel<<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const double2*>(grid_in),
+                                                        reinterpret_cast<double2*>(grid_out), p->sl, p->nang, p->nx,
+                                                        p->tab, p->fltb);
   SPI_TRY(check_kernel("fs_normal64_kernel"));
   p->ctx->count(2);
   return 0;
@@ -763,27 +590,59 @@ int spi_fslice_normal64(const spi_fslice_plan* p, const double* grid_in, double 
 int spi_fslice_forward64(const spi_fslice_plan* p, const double* grid, double* slices, void* stream) {
   if (!p || !grid || !slices) return fail(kInvalid, "spi_fslice_forward64: NULL argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  fs_extract64_kernel<<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const double2*>(grid),
-                                                         reinterpret_cast<double2*>(slices), p->sl, p->nang, p->nx,
-                                                         p->tab, p->fltb);
-  SPI_TRY(check_kernel("fs_extract64_kernel"));
-  p->ctx->count();
-  return 0;
+  return fs_extract<double2>(p, grid, slices, 0, p->nang, s);
 }
 
 int spi_fslice_adjoint64(const spi_fslice_plan* p, const float* slices, double* grid, void* stream) {
   if (!p || !grid || !slices) return fail(kInvalid, "spi_fslice_adjoint64: NULL argument");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  SPI_CUDA(cudaMemsetAsync(grid, 0, fs_grid_elems(p) * sizeof(double2), s));
-  if (fs_w8())
-    fs_insert64w_kernel<<<fs_blocks(p), 256, kFsSmem, s>>>(reinterpret_cast<const float2*>(slices), grid, p->sl,
-                                                           p->nang, p->nx, p->tab, p->fltb);
+  return fs_adjoint<SlabFs64>(p, slices, grid, sizeof(double2), s);
+}
+
+int spi_fslice_normal_ws_bytes(const spi_fslice_plan* p, int fp64, long long* bytes) {
+  if (!p || !bytes) return fail(kInvalid, "spi_fslice_normal_ws_bytes: NULL argument");
+  const long long per = (long long)fs_plane(p) * (fp64 ? sizeof(double2) : sizeof(float2));
+  // about 128 MB of slices: 242 of 128^3 in FP64, 0.6 ms of work per pair of launches
+  const long long chunk = std::max(1LL, std::min<long long>(p->nang, (128LL << 20) / per));
+  *bytes = per * chunk + fs_counter_bytes(p, chunk);
+  return 0;
+}
+
+int spi_fslice_normal_ws(const spi_fslice_plan* p, const void* grid_in, double lam, void* grid_out, int fp64, void* ws,
+                         long long ws_bytes, void* stream) {
+  if (!p || !grid_in || !grid_out || !ws) return fail(kInvalid, "spi_fslice_normal_ws: NULL argument");
+  if (grid_in == grid_out) return fail(kInvalid, "spi_fslice_normal_ws: input and output must differ");
+  const long long per = (long long)fs_plane(p) * (fp64 ? sizeof(double2) : sizeof(float2));
+  // as many slices as fit beside one work counter per insertion launch
+  long long chunk = std::min<long long>(p->nang, ws_bytes / per);
+  while (chunk > 0 && chunk * per + fs_counter_bytes(p, chunk) > ws_bytes) --chunk;
+  if (chunk < 1)
+    return fail(kInvalid, "spi_fslice_normal_ws: workspace of %lld bytes, one slice and the counters take %lld", ws_bytes,
+                per + fs_counter_bytes(p, 1));
+  if (reinterpret_cast<uintptr_t>(ws) % 16)
+    return fail(kInvalid, "spi_fslice_normal_ws: the workspace must be 16-byte aligned");
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const size_t ne = fs_grid_elems(p);
+  if (fp64)
+    fs_scale64_kernel<<<fs_grid_blocks(p, ne), 256, 0, s>>>(static_cast<const double2*>(grid_in), lam,
+                                                            static_cast<double2*>(grid_out), ne);
   else
-    fs_normal64_kernel<false><<<fs_blocks(p), 256, kFsSmem, s>>>(nullptr, reinterpret_cast<const float2*>(slices),
-                                                                 reinterpret_cast<double2*>(grid), p->sl, p->nang,
-                                                                 p->nx, p->tab, p->fltb);
-  SPI_TRY(check_kernel("fs_normal64_kernel<insert>"));
+    fs_scale_kernel<<<fs_grid_blocks(p, ne), 256, 0, s>>>(static_cast<const float2*>(grid_in), (float)lam,
+                                                          static_cast<float2*>(grid_out), ne);
+  SPI_TRY(check_kernel("fs_scale_kernel"));
   p->ctx->count();
+  auto* work = reinterpret_cast<unsigned long long*>(static_cast<char*>(ws) + chunk * per);
+  SPI_CUDA(cudaMemsetAsync(work, 0, (size_t)fs_counter_bytes(p, chunk), s));
+  for (int a = 0; a < p->nang; a += (int)chunk, ++work) {
+    const int n = std::min((int)chunk, p->nang - a);
+    if (fp64) {
+      SPI_TRY((fs_extract<double2>(p, grid_in, ws, a, n, s)));
+      SPI_TRY(fs_insert<SlabFs64d>(p, ws, grid_out, a, n, work, s));
+    } else {
+      SPI_TRY((fs_extract<float2>(p, grid_in, ws, a, n, s)));
+      SPI_TRY(fs_insert<SlabFs>(p, ws, grid_out, a, n, work, s));
+    }
+  }
   return 0;
 }
 

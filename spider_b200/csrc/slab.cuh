@@ -1,6 +1,6 @@
 // Column insertion of central slices (ONELINE, oneline.f:38-200) on sm_100a.
-// Included by bp.cu after SliceDesc, load_spec and red_add_v4; the geometry
-// is in slab_geom.h.
+// Used by bp.cu (grids of {Re X, Im X, W, 0}) and fslice.cu (complex grids in
+// FP32 and FP64, without W); the geometry is in slab_geom.h.
 //
 // A form that adds every tap with its own 16-byte L2 reduction (47 taps per
 // pixel, 13 of one slice on every voxel, four lanes per pixel over the four
@@ -29,19 +29,69 @@
 // at a time, which leaves registers for four CTAs per SM (8.8 with three).
 #pragma once
 
+#include <cuda_bf16.h>
+
+#include <type_traits>
+
 #include "slab_geom.h"
 
 namespace spi {
 
+struct SliceDesc {
+  float dm[6];  // DMS(1:6): first two columns of the (symmetrised) rotation
+  int img;      // index of the slice's values in the launch
+  int grid;     // target grid (BP 32F half set)
+};
+static_assert(sizeof(SliceDesc) == 32, "slice descriptor is 32 bytes");
+
+// What a column insertion reads and adds: slice values of type Raw, a weight
+// grid or not, sums in FP32 or FP64.
+template <class Raw_, bool W_, bool D_>
+struct SlabForm {
+  using Raw = Raw_;
+  static constexpr bool W = W_, D = D_;
+};
+using SlabBp = SlabForm<float2, true, false>;              // float4 grid {Re X, Im X, W, 0}
+using SlabBpBf16 = SlabForm<__nv_bfloat162, true, false>;  // the same from BF16 spectra
+using SlabFs = SlabForm<float2, false, false>;             // float2 grid
+using SlabFs64 = SlabForm<float2, false, true>;            // double2 grid from FP32 slices
+using SlabFs64d = SlabForm<double2, false, true>;          // double2 grid from FP64 slices
+
+// G[i] += v as one 16-byte reduction in L2 (red.global.add.v4.f32).  The
+// address is converted to the global window explicitly: the kernel takes its
+// grid pointer from shared memory, and on such a generic pointer
+// atomicAdd(float4*) was not compiled to the vector reduction (measured:
+// 1.9x the instructions and no L2 reduction requests).
+__device__ __forceinline__ void red_add_v4(float4* p, float4 v) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(p)), "f"(v.x),
+               "f"(v.y), "f"(v.z), "f"(v.w));
+}
+// voxel i of the form's grid += (re, im) and its weight
+template <class F>
+__device__ __forceinline__ void slab_red(void* grid, size_t i, float re, float im, float w) {
+  if (F::W) {
+    red_add_v4(static_cast<float4*>(grid) + i, make_float4(re, im, w, 0.0f));
+  } else {
+    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(__cvta_generic_to_global(static_cast<float2*>(grid) + i)),
+                 "f"(re), "f"(im));
+  }
+}
+__device__ __forceinline__ void slab_red64(void* grid, size_t i, double re, double im) {
+  const auto a = __cvta_generic_to_global(static_cast<double2*>(grid) + i);
+  asm volatile("red.global.add.f64 [%0], %1;" ::"l"(a), "d"(re));
+  asm volatile("red.global.add.f64 [%0+8], %1;" ::"l"(a), "d"(im));
+}
+
 constexpr int kSlabMaxClass = 16;
 constexpr int kSlabThreads = kSlabTile * kSlabTile / 2;   // consumers: two columns each, neighbours along v
 constexpr int kSlabBlocks = 4;                            // CTAs per SM (96 registers, 50 KB each)
+constexpr int kSlabBlocks64 = 3;                          // the same with FP64 sums (128 registers, 50-60 KB)
 
 struct SlabClass {
   const void* spec;            // spectra of the class's images in this launch
   const SliceDesc* slices;
-  float4* g0;                  // grids the taps go to (half-set 1 and 2)
-  float4* g1;
+  void* g0;                    // grids the taps go to (half-set 1 and 2)
+  void* g1;
   const float* tab;            // interpolation table (5,000 entries)
   long long item0;             // first work item of the class
   int nx, nslices;
@@ -57,19 +107,19 @@ struct SlabArgs {
 // A tile as the producer warp hands it over
 struct SlabTile {
   SlabFrame f;
-  float4* g;                   // grid of its slice
+  void* g;                     // grid of its slice
   float fltb;
   int banks;                   // 0: no tile is left
   int u0, v0, jlo, nr, nx, cls;
   int4 rows[kSlabRows];        // {first staged pixel - lo, lo, hi, 0}
 };
-template <bool BF16>
+template <class F>
 struct SlabSmem {
-  float4 pix[kSlabPix];        // {u, v, Re, Im}
+  typename std::conditional<F::D, float2, float4>::type pix[kSlabPix];   // {u, v, Re, Im}; FP64: {u, v}, the value in raw
   float4 t[kSlabPix];          // weights along w by residue modulo 4
-  int code[kSlabPix];          // slab_masks, kSlabMate
+  int code[kSlabPix];          // slab_masks, kSlabMate, kSlabRep
   SlabTile tile[2];
-  typename std::conditional<BF16, __nv_bfloat162, float2>::type raw[2][kSlabPix];   // spectrum values
+  typename F::Raw raw[2][kSlabPix];   // slice values
   float tab[kSlabTab];
 };
 
@@ -121,13 +171,18 @@ __device__ __forceinline__ void slab_setup(SlabTile& T, const SlabFrame& f, int 
   }
 }
 
-// 8 (4) bytes from global to shared memory, asynchronously
+// 4, 8 or 16 bytes from global to shared memory, asynchronously
 __device__ __forceinline__ void slab_copy(float2* dst, const float2* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
 __device__ __forceinline__ void slab_copy(__nv_bfloat162* dst, const __nv_bfloat162* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
 }
+__device__ __forceinline__ void slab_copy(double2* dst, const double2* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ double2 slab_double2(float2 v) { return make_double2(v.x, v.y); }
+__device__ __forceinline__ double2 slab_double2(double2 v) { return v; }
 __device__ __forceinline__ float2 slab_float2(float2 v) { return v; }
 __device__ __forceinline__ float2 slab_float2(__nv_bfloat162 v) { return make_float2(__low2float(v), __high2float(v)); }
 
@@ -149,6 +204,7 @@ __device__ __forceinline__ void slab_fetch(V* raw, const SlabTile& T, const V* s
 }
 
 constexpr int kSlabMate = 1;   // not the canonical pixel of its pair
+constexpr int kSlabRep = 2;    // the stored pixel of its pair
 
 // Which residues of a window that starts at w lie in which bank.  Two banks:
 // the sign of byte r says whether the window's voxel of residue r modulo 4
@@ -189,21 +245,24 @@ __device__ __forceinline__ void slab_spread(const float4& t, int m, unsigned lon
 }
 
 // The origin is its own mate: its reflected taps, x = -1 to x = 1, go out
-// apart, once per slice.  br, bi: its value.
-__device__ __noinline__ void slab_origin(const float* tab, float fltb, float4* __restrict__ G, int nx, float br, float bi) {
+// apart, once per slice.  b: its value.
+template <class F>
+__device__ __noinline__ void slab_origin(const float* tab, float fltb, void* G, int nx, double2 b) {
   const float w0 = tab[0], w1 = tab[slab_tab_index(0.0f, 1, fltb, kSlabTab - 1)];
   const int N = 2 * nx;
   for (int e = 0; e < 9; ++e) {
     const int y = e % 3 - 1, z = e / 3 - 1;
     const float wg = __fmul_rn(w1, __fmul_rn(y ? w1 : w0, z ? w1 : w0));
-    red_add_v4(G + ((size_t)(z < 0 ? N + z : z) * N + (y < 0 ? N + y : y)) * (size_t)(nx + 1) + 1,
-               make_float4(__fmul_rn(br, wg), -__fmul_rn(bi, wg), wg, 0.0f));
+    const size_t i = ((size_t)(z < 0 ? N + z : z) * N + (y < 0 ? N + y : y)) * (size_t)(nx + 1) + 1;
+    if (F::D) slab_red64(G, i, __dmul_rn(b.x, (double)wg), -__dmul_rn(b.y, (double)wg));
+    else slab_red<F>(G, i, __fmul_rn((float)b.x, wg), -__fmul_rn((float)b.y, wg), wg);
   }
 }
 
 // The taps of a pixel whose value is not finite on the tile's columns, one by
 // one: its products with zero weights, which slab_gather forms, would not be zero.
-__device__ __noinline__ void slab_direct(const float* tab, const SlabTile& T, const SlabPix& p, float br, float bi) {
+template <class F>
+__device__ __noinline__ void slab_direct(const float* tab, const SlabTile& T, const SlabPix& p, double2 b) {
   const int nx = T.nx, N = 2 * nx;
   const int fu = slab_first(p.u), fv = slab_first(p.v), fw = slab_first(p.w);
   auto tap = [&](float c, int k) { return tab[slab_tab_index(c, k, T.fltb, kSlabTab - 1)]; };
@@ -214,14 +273,15 @@ __device__ __noinline__ void slab_direct(const float* tab, const SlabTile& T, co
     if (x < 0 || (x == 0 && !p.canon)) continue;
     const float wg = __fmul_rn(tap(p.u, u), __fmul_rn(tap(p.v, v), tap(p.w, w)));
     if (wg == 0.0f) continue;
-    red_add_v4(T.g + ((size_t)(z < 0 ? N + z : z) * N + (y < 0 ? N + y : y)) * (size_t)(nx + 1) + x,
-               make_float4(__fmul_rn(br, wg), __fmul_rn(bi, wg), 0.0f, 0.0f));
+    const size_t i = ((size_t)(z < 0 ? N + z : z) * N + (y < 0 ? N + y : y)) * (size_t)(nx + 1) + x;
+    if (F::D) slab_red64(T.g, i, __dmul_rn(b.x, (double)wg), __dmul_rn(b.y, (double)wg));
+    else slab_red<F>(T.g, i, __fmul_rn((float)b.x, wg), __fmul_rn((float)b.y, wg), 0.0f);
   }
 }
 
 // The tile's pixels into the form that slab_gather reads: eight lanes per row
-template <int NB, bool BF16>
-__device__ __forceinline__ void slab_stage(SlabSmem<BF16>& S, const SlabTile& T, const SlabFrame& f, int buf) {
+template <int NB, class F>
+__device__ __forceinline__ void slab_stage(SlabSmem<F>& S, const SlabTile& T, const SlabFrame& f, int buf) {
   const int nx = T.nx, jlo = T.jlo, nr = T.nr, l8 = threadIdx.x & 7;
   const float fltb = T.fltb;
   for (int r = threadIdx.x >> 3; r < nr; r += kSlabThreads / 8) {
@@ -232,16 +292,32 @@ __device__ __forceinline__ void slab_stage(SlabSmem<BF16>& S, const SlabTile& T,
       const int q = row.x + I;
       const SlabPix p = slab_pixel(f, I, J);
       if (!slab_inside(f, p, I, J, nx)) {   // adds nothing
-        S.pix[q] = make_float4(p.u, p.v, 0.0f, 0.0f);
+        if constexpr (F::D) {
+          S.pix[q] = make_float2(p.u, p.v);
+          S.raw[buf][q] = typename F::Raw{0, 0};
+        } else {
+          S.pix[q] = make_float4(p.u, p.v, 0.0f, 0.0f);
+        }
         S.t[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         S.code[q] = 0;
         continue;
       }
       // SPIDER forward sign = conjugate of the cuFFT R2C output; conjugated again for a mate
-      const float2 sp = slab_float2(S.raw[buf][q]);
-      const float bi = p.rep ? -sp.y : sp.y;
-      const bool fin = isfinite(sp.x) && isfinite(bi);
-      S.pix[q] = make_float4(p.u, p.v, fin ? sp.x : 0.0f, fin ? bi : 0.0f);
+      double2 val;
+      bool fin;
+      if constexpr (F::D) {
+        const typename F::Raw sp = S.raw[buf][q];
+        val = make_double2(sp.x, p.rep ? -sp.y : sp.y);
+        fin = isfinite(sp.x) && isfinite(sp.y);
+        S.pix[q] = make_float2(p.u, p.v);
+        if (!fin) S.raw[buf][q] = typename F::Raw{0, 0};
+      } else {
+        const float2 sp = slab_float2(S.raw[buf][q]);
+        const float bi = p.rep ? -sp.y : sp.y;
+        val = make_double2(sp.x, bi);
+        fin = isfinite(sp.x) && isfinite(bi);
+        S.pix[q] = make_float4(p.u, p.v, fin ? sp.x : 0.0f, fin ? bi : 0.0f);
+      }
       const int fw = slab_first(p.w);
       float tw[4];
 #pragma unroll
@@ -253,26 +329,59 @@ __device__ __forceinline__ void slab_stage(SlabSmem<BF16>& S, const SlabTile& T,
       const bool s1 = fw & 1, s2 = fw & 2;
       const float a0 = s1 ? tw[3] : tw[0], a1 = s1 ? tw[0] : tw[1], a2 = s1 ? tw[1] : tw[2], a3 = s1 ? tw[2] : tw[3];
       S.t[q] = make_float4(s2 ? a2 : a0, s2 ? a3 : a1, s2 ? a0 : a2, s2 ? a1 : a3);
-      S.code[q] = slab_masks<NB>(fw) | (p.canon ? 0 : kSlabMate);
-      if (!fin) slab_direct(S.tab, T, p, sp.x, bi);
+      S.code[q] = slab_masks<NB>(fw) | (p.canon ? 0 : kSlabMate) | (p.rep ? kSlabRep : 0);
+      if (!fin) slab_direct<F>(S.tab, T, p, val);
       if (I == 0 && J == 0 && T.u0 <= 0 && T.u0 + kSlabTile > 0 && T.v0 <= 0 && T.v0 + kSlabTile > 0)
-        slab_origin(S.tab, fltb, T.g, nx, sp.x, bi);
+        slab_origin<F>(S.tab, fltb, T.g, nx, val);
     }
   }
+}
+
+// Voxels of one column by residue
+struct SlabCol {
+  int base, res, N;      // first voxel along w, its residue
+  bool wx;               // w is x: no voxels below zero (the mate's taps)
+  unsigned at0, step;    // voxel at w = 0 and the stride along w (grids hold < 2^32 voxels)
+  template <int NB>
+  __device__ __forceinline__ long long voxel(int j) const {   // of residue j; -1: none
+    int off = j - res;
+    if (off < 0) off += 4 * NB;
+    int k = base + off;
+    if (k < 0) {
+      if (wx) return -1;
+      k += N;
+    }
+    return (long long)(at0 + (unsigned)k * step);
+  }
+};
+template <int NB>
+__device__ __forceinline__ SlabCol slab_col(const SlabFrame& f, int nx, int U, int V) {
+  SlabCol c;
+  const unsigned rl = (unsigned)(nx + 1), N = 2u * (unsigned)nx;
+  const unsigned iv = (unsigned)(V >= 0 ? V : (int)N + V);
+  c.base = slab_col_base(f, (float)U, (float)V);
+  c.res = slab_residue(c.base, NB);
+  c.N = (int)N;
+  c.wx = f.d == 0;
+  if (f.d == 2) { c.at0 = iv * rl + (unsigned)U; c.step = N * rl; }
+  else if (f.d == 1) { c.at0 = iv * N * rl + (unsigned)U; c.step = rl; }
+  else { c.at0 = (iv * N + (unsigned)(U >= 0 ? U : (int)N + U)) * rl; c.step = 1u; }
+  return c;
 }
 
 // Columns (U, V) .. (U, V + NC - 1): walk the pixels that reach them, keep the
 // sums by residue in registers (pairs of residues 2 j, 2 j + 1 of Re X, Im X, W),
 // and add them to the grid.
-template <int NC, int NB, bool BF16>
-__device__ __forceinline__ void slab_gather(const SlabSmem<BF16>& S, const SlabTile& T, const SlabFrame& f, int U, int V) {
+template <int NC, int NB, class F>
+__device__ __forceinline__ void slab_gather(const SlabSmem<F>& S, const SlabTile& T, const SlabFrame& f, int U, int V) {
   const int nx = T.nx, jlo = T.jlo;
   const float fltb = T.fltb, u = (float)U, v = (float)V;
-  unsigned long long acc[NC][3][2 * NB];
+  constexpr int kSums = F::W ? 3 : 2;
+  unsigned long long acc[NC][kSums][2 * NB];
 #pragma unroll
   for (int c = 0; c < NC; ++c)
 #pragma unroll
-    for (int e = 0; e < 3; ++e)
+    for (int e = 0; e < kSums; ++e)
 #pragma unroll
       for (int j = 0; j < 2 * NB; ++j) acc[c][e][j] = 0ull;
   const int mate = (f.d != 0 && U == 0) ? kSlabMate : 0;   // column x = 0 takes the canonical pixels only
@@ -289,7 +398,7 @@ __device__ __forceinline__ void slab_gather(const SlabSmem<BF16>& S, const SlabT
       for (int j = 0; j < 2 * NB; ++j) {
         slab_fma2(acc[c][0][j], re2, tt[j]);
         slab_fma2(acc[c][1][j], im2, tt[j]);
-        slab_fma2(acc[c][2][j], w2, tt[j]);
+        if (F::W) slab_fma2(acc[c][kSums - 1][j], w2, tt[j]);
       }
     }
   };
@@ -321,69 +430,137 @@ __device__ __forceinline__ void slab_gather(const SlabSmem<BF16>& S, const SlabT
       b = bn; t = tn; code = coden; q = qn;
     }
   }
-  const int N = 2 * nx;
-  const unsigned rl = (unsigned)(nx + 1);
-  float4* G = T.g;
 #pragma unroll
   for (int c = 0; c < NC; ++c) {
-    const int Vc = V + c;
-    const int base = slab_col_base(f, u, v + (float)c), res = slab_residue(base, NB);
-    const unsigned iv = (unsigned)(Vc >= 0 ? Vc : N + Vc);
-    unsigned col, step;   // voxel of the column at w = 0 and the stride along w (grids hold < 2^32 voxels)
-    if (f.d == 2) { col = iv * rl + (unsigned)U; step = (unsigned)N * rl; }
-    else if (f.d == 1) { col = iv * (unsigned)N * rl + (unsigned)U; step = rl; }
-    else { col = (iv * (unsigned)N + (unsigned)(U >= 0 ? U : N + U)) * rl; step = 1u; }
+    const SlabCol col = slab_col<NB>(f, nx, U, V + c);
 #pragma unroll
     for (int j = 0; j < 2 * NB; ++j) {
-      const float2 re = slab_unpack(acc[c][0][j]), im = slab_unpack(acc[c][1][j]), w = slab_unpack(acc[c][2][j]);
+      const float2 re = slab_unpack(acc[c][0][j]), im = slab_unpack(acc[c][1][j]), w = slab_unpack(acc[c][kSums - 1][j]);
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const float wg = e ? w.y : w.x;
-        if (wg == 0.0f) continue;
-        int off = 2 * j + e - res;
-        if (off < 0) off += 4 * NB;
-        int k = base + off;
-        if (k < 0) {
-          if (f.d == 0) continue;   // x < 0: the mate's taps
-          k += N;
-        }
-        red_add_v4(G + (size_t)(col + (unsigned)k * step), make_float4(e ? re.y : re.x, e ? im.y : im.x, wg, 0.0f));
+        const float r = e ? re.y : re.x, i = e ? im.y : im.x, wg = e ? w.y : w.x;
+        if (F::W ? wg == 0.0f : r == 0.0f && i == 0.0f) continue;
+        const long long vx = col.voxel<NB>(2 * j + e);
+        if (vx >= 0) slab_red<F>(T.g, (size_t)vx, r, i, wg);
       }
     }
   }
 }
 
+// The same with FP64 sums, one column: every tap's weight is the FP32 product
+// TX * (TY * TZ) of the per-tap form, bit for bit, taken into FP64.
+template <int NB, class F>
+__device__ __forceinline__ void slab_gather64(const SlabSmem<F>& S, const SlabTile& T, const SlabFrame& f, int buf, int U,
+                                              int V) {
+  const int nx = T.nx, jlo = T.jlo;
+  const float fltb = T.fltb, u = (float)U, v = (float)V;
+  double re[4 * NB], im[4 * NB];
+#pragma unroll
+  for (int j = 0; j < 4 * NB; ++j) re[j] = im[j] = 0.0;
+  const int mate = (f.d != 0 && U == 0) ? kSlabMate : 0;   // column x = 0 takes the canonical pixels only
+  const bool wx = f.d == 0;                                // w is x: TX is the weight along w
+  auto tap = [&](float p, float k) { return S.tab[slab_nint(__fmul_rn(fabsf(__fsub_rn(p, k)), fltb))]; };
+  int r0, r1;
+  slab_block_rows(f, u, v, 1, 1, jlo, T.nr, r0, r1);
+  for (int r = r0; r <= r1; ++r) {
+    const int4 row = T.rows[r];
+    float fl, fh;
+    slab_span(f, u, v, kSlabR, kSlabR, jlo + r, fl, fh);
+    const int i0 = slab_ceil(fmaxf(fl, (float)row.y)), i1 = slab_floor(fminf(fh, (float)row.z));
+    if (i0 > i1) continue;
+    // the next pixel's reads and weights are under way while this one's products are added
+    int q = row.x + i0;
+    const int q1 = row.x + i1;
+    float2 b = S.pix[q];
+    float4 t = S.t[q];
+    int code = S.code[q];
+    double2 x = slab_double2(S.raw[buf][q]);
+    float wu = tap(b.x, u), wv = tap(b.y, v);
+    for (;;) {
+      const int qn = min(q + 1, q1);
+      const float2 bn = S.pix[qn];
+      const float4 tn = S.t[qn];
+      const int coden = S.code[qn];
+      const double2 xn = slab_double2(S.raw[buf][qn]);
+      if (code & mate) wu = 0.0f;
+      const double xi = code & kSlabRep ? -x.y : x.y;
+      const float tr[4] = {t.x, t.y, t.z, t.w};
+      const float uv = __fmul_rn(wu, wv);
+      int k[4];
+      if (NB == 2) {
+        k[0] = slab_sign<0x8888>(code); k[1] = slab_sign<0x9999>(code);
+        k[2] = slab_sign<0xaaaa>(code); k[3] = slab_sign<0xbbbb>(code);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const double d = (double)(wx ? __fmul_rn(tr[e], uv) : __fmul_rn(wu, __fmul_rn(wv, tr[e])));
+        if (NB == 2) {
+          const int hi = __double2hiint(d), lo = __double2loint(d);
+          const double d0 = __hiloint2double(hi & k[e], lo & k[e]), d1 = __hiloint2double(hi & ~k[e], lo & ~k[e]);
+          re[e] = fma(x.x, d0, re[e]);
+          im[e] = fma(xi, d0, im[e]);
+          re[4 + e] = fma(x.x, d1, re[4 + e]);
+          im[4 + e] = fma(xi, d1, im[4 + e]);
+        } else {
+#pragma unroll
+          for (int n = 0; n < NB; ++n) {
+            if (code & (256 << (4 * n + e))) {
+              re[4 * n + e] = fma(x.x, d, re[4 * n + e]);
+              im[4 * n + e] = fma(xi, d, im[4 * n + e]);
+            }
+          }
+        }
+      }
+      if (q >= q1) break;
+      wu = tap(bn.x, u);
+      wv = tap(bn.y, v);
+      b = bn; t = tn; code = coden; x = xn; q = qn;
+    }
+  }
+  const SlabCol col = slab_col<NB>(f, nx, U, V);
+#pragma unroll
+  for (int j = 0; j < 4 * NB; ++j) {
+    if (re[j] == 0.0 && im[j] == 0.0) continue;
+    const long long vx = col.voxel<NB>(j);
+    if (vx >= 0) slab_red64(T.g, (size_t)vx, re[j], im[j]);
+  }
+}
+
 // One tile of one slice, by the consumer warps
-template <int NB, bool BF16>
-__device__ __forceinline__ void slab_tile(SlabSmem<BF16>& S, const SlabTile& T, int buf) {
+template <int NB, class F>
+__device__ __forceinline__ void slab_tile(SlabSmem<F>& S, const SlabTile& T, int buf) {
   const SlabFrame f = T.f;
-  slab_stage<NB, BF16>(S, T, f, buf);
+  slab_stage<NB, F>(S, T, f, buf);
   slab_bar<2>(kSlabThreads);
-  // Steep slices (three banks) take a thread's two columns one after the other: as
-  // many operations as together, and their sums fit the registers.
+  // Steep slices (three banks) and FP64 sums take a thread's two columns one after the
+  // other: about as many operations as together, and their sums fit the registers.
   const int U = T.u0 + (threadIdx.x & 15), V = T.v0 + 2 * (threadIdx.x >> 4);
-  if (NB == 2) {
-    slab_gather<2, NB, BF16>(S, T, f, U, V);
+  if constexpr (F::D) {
+#pragma unroll 1
+    for (int c = 0; c < 2; ++c) slab_gather64<NB, F>(S, T, f, buf, U, V + c);
+  } else if (NB == 2) {
+    slab_gather<2, NB, F>(S, T, f, U, V);
   } else {
 #pragma unroll 1
-    for (int c = 0; c < 2; ++c) slab_gather<1, NB, BF16>(S, T, f, U, V + c);
+    for (int c = 0; c < 2; ++c) slab_gather<1, NB, F>(S, T, f, U, V + c);
   }
 }
 
 // A CTA is one producer warp and kSlabThreads consumers.  The producer takes
 // work items (a slice's row of tiles along u, or every `parts`-th tile of it
-// when a launch has few slices) in slice-major order from one counter and
-// prepares tile k + 1 -- its frame, rows and the copies of its spectrum values
-// -- while the consumers stage and gather tile k.  The two meet once per tile.
-template <bool BF16>
-__global__ void __launch_bounds__(kSlabThreads + 32, kSlabBlocks) insert_x4_kernel(const __grid_constant__ SlabArgs P,
-                                                                                  unsigned long long* __restrict__ work) {
+// when a launch has few slices) in slice-major order and prepares tile k + 1
+// -- its frame, rows and the copies of its slice values -- while the consumers
+// stage and gather tile k.  The two meet once per tile.  `work`: a counter of
+// the launch, zero at its start (a grid stride over the items instead left the
+// SMs idle for a quarter of 240 slices at 128^3: rows differ in length).
+template <class F>
+__device__ __forceinline__ void slab_main(const SlabArgs& P, unsigned long long* __restrict__ work) {
   extern __shared__ __align__(16) unsigned char slab_raw[];
-  SlabSmem<BF16>& S = *reinterpret_cast<SlabSmem<BF16>*>(slab_raw);
+  SlabSmem<F>& S = *reinterpret_cast<SlabSmem<F>*>(slab_raw);
   const int tid = threadIdx.x;
   if (tid >= kSlabThreads) {
     const int lane = tid - kSlabThreads;
-    using V = typename std::conditional<BF16, __nv_bfloat162, float2>::type;
+    using V = typename F::Raw;
     int buf = 0;
     unsigned long long next = 0;   // the item after the current one
     if (lane == 0) next = atomicAdd(work, 1ull);
@@ -440,9 +617,34 @@ __global__ void __launch_bounds__(kSlabThreads + 32, kSlabBlocks) insert_x4_kern
       for (int i = tid; i < kSlabTab; i += kSlabThreads) S.tab[i] = P.cls[have].tab[i];
       slab_bar<2>(kSlabThreads);
     }
-    if (T.banks == 2) slab_tile<2, BF16>(S, T, buf);
-    else slab_tile<3, BF16>(S, T, buf);
+    if (T.banks == 2) slab_tile<2, F>(S, T, buf);
+    else slab_tile<3, F>(S, T, buf);
   }
+}
+
+// BP 3F / BP 32F
+template <class F>
+__global__ void __launch_bounds__(kSlabThreads + 32, kSlabBlocks) insert_x4_kernel(const __grid_constant__ SlabArgs P,
+                                                                                unsigned long long* __restrict__ work) {
+  slab_main<F>(P, work);
+}
+
+// Work items of the classes: a slice's row of tiles each, or its parts when
+// all rows together would give the launch's `blocks` CTAs fewer than eight
+// items (the tail of a launch is about half an item per CTA: 200 slices at
+// 64^3 0.148 against 0.176 ms with whole rows).  Returns their number.
+inline long long slab_items(long long blocks, SlabClass* cls, int ncls) {
+  auto rows_of = [](const SlabClass& m) { return (long long)m.nslices * ((2 * m.nx + kSlabTile - 1) / kSlabTile); };
+  long long rows = 0, items = 0;
+  for (int k = 0; k < ncls; ++k) rows += rows_of(cls[k]);
+  for (int k = 0; k < ncls; ++k) {
+    const long long most = (cls[k].nx + kSlabTile - 1) / kSlabTile;
+    const long long parts = rows > 0 ? (8 * blocks + rows - 1) / rows : 1;
+    cls[k].parts = (int)(parts < 1 ? 1 : parts < most ? parts : most);
+    cls[k].item0 = items;
+    items += rows_of(cls[k]) * cls[k].parts;
+  }
+  return items;
 }
 
 }  // namespace spi
