@@ -1631,6 +1631,8 @@ void bp_release(spi_ctx* c) {
   for (auto& g : c->comp) g.release();
   c->unfolded = 0;
   c->comp_dirty = false;
+  c->virgin = false;
+  for (int g = 0; g < 2; ++g) c->part_zero[g] = c->comp_zero[g] = false;
   c->gptr[0] = c->gptr[1] = nullptr;
   c->wkb_nx = 0;
   c->imgs.release();
@@ -1672,7 +1674,12 @@ static size_t grid_voxels(const spi_ctx* c) { return (size_t)(c->nx + 1) * c->n 
 
 // The grid the insertion adds into: the partial grid with compensated
 // accumulation, else the grid itself.
-static float4* insert_target(spi_ctx* c, int g) { return c->accum ? c->part[g].as<float4>() : c->gptr[g]; }
+// fold_grids may exchange the two, so it is asked anew for every launch.
+static float4* insert_target(spi_ctx* c, int g) {
+  if (!c->accum) return c->gptr[g];
+  c->part_zero[g] = false;
+  return c->part[g].as<float4>();
+}
 
 // Fold the partial grids into the grids (two-sum, compensation kept), or with
 // `collapse` also add the compensation into the grids and clear it; a no-op
@@ -1680,6 +1687,19 @@ static float4* insert_target(spi_ctx* c, int g) { return c->accum ? c->part[g].a
 static int fold_grids(spi_ctx* c, bool collapse) {
   if (!c->accum || c->ngrids == 0) return 0;
   if (c->unfolded == 0 && !(collapse && c->comp_dirty)) return 0;
+  if (c->virgin) {
+    // The first fold of library-owned grids: grid and compensation are still all
+    // zero, so the partial sums ARE the grid (a two-sum with zero is exact) and the
+    // zero grid is the next partial one.  1.4 ms of a fold of two 256^3 grids.
+    for (int g = 0; g < c->ngrids; ++g) {
+      std::swap(c->grid[g], c->part[g]);
+      c->gptr[g] = c->grid[g].as<float4>();
+      c->part_zero[g] = true;
+    }
+    c->virgin = false;
+    c->unfolded = 0;
+    return 0;
+  }
   const size_t nvox = grid_voxels(c);
   int ev = c->phase_begin(8);
   for (int g = 0; g < c->ngrids; ++g) {
@@ -1694,6 +1714,10 @@ static int fold_grids(spi_ctx* c, bool collapse) {
   c->phase_end(ev);
   c->unfolded = 0;
   c->comp_dirty = !collapse;
+  for (int g = 0; g < c->ngrids; ++g) {   // fold_kernel clears the partial grid and, collapsing, the compensation
+    c->part_zero[g] = true;
+    c->comp_zero[g] = collapse;
+  }
   return 0;
 }
 
@@ -1875,6 +1899,17 @@ int spi_ctx_timing(spi_ctx* c, double* ms_out, long long* count_out) {
 }
 long long spi_ctx_device_bytes(const spi_ctx* c) { return c ? c->device_bytes() : 0; }
 
+// A buffer of `bytes` zero bytes; `zero` says whether it is known to be one
+// already (a same-size open after a finished reconstruction: folds leave the
+// partial and the collapsed compensation grids zero).
+static int zeroed(spi_ctx* c, DevBuf& b, size_t bytes, bool& zero) {
+  if (b.bytes < bytes) zero = false;
+  SPI_TRY(b.ensure(bytes));
+  if (!zero) SPI_CUDA(cudaMemsetAsync(b.p, 0, bytes, c->stream));
+  zero = true;
+  return 0;
+}
+
 int spi_bp_open(spi_ctx* c, int nx, int ngrids, const float* sym_angles, int nsym) {
   if (!c) return fail(kInvalid, "spi_bp_open: NULL context");
   if (nx < 8 || nx > 512) return fail(kInvalid, "spi_bp_open: nx = %d must be 8..512", nx);
@@ -1910,12 +1945,11 @@ int spi_bp_open(spi_ctx* c, int nx, int ngrids, const float* sym_angles, int nsy
     }
     SPI_CUDA(cudaMemsetAsync(c->gptr[g], 0, gbytes, c->stream));
     if (c->accum) {
-      SPI_TRY(c->part[g].ensure(gbytes));
-      SPI_TRY(c->comp[g].ensure(gbytes));
-      SPI_CUDA(cudaMemsetAsync(c->part[g].p, 0, gbytes, c->stream));
-      SPI_CUDA(cudaMemsetAsync(c->comp[g].p, 0, gbytes, c->stream));
+      SPI_TRY(zeroed(c, c->part[g], gbytes, c->part_zero[g]));
+      SPI_TRY(zeroed(c, c->comp[g], gbytes, c->comp_zero[g]));
     }
   }
+  c->virgin = c->accum && !c->ext_grid[0] && (ngrids == 1 || !c->ext_grid[1]);
   c->unfolded = 0;
   c->comp_dirty = false;
   if (c->fold_every <= 0) c->fold_every = env_int("SPI_BP_FOLD", 4096);
@@ -2460,7 +2494,6 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
     SPI_CUDA(cudaStreamWaitEvent(cs, c->ev_fork, 0));
   }
   std::vector<char> done_valid(nsubs, 0);
-  float4* g1 = insert_target(c, c->ngrids == 2 ? 1 : 0);
   for (int a0 = 0; a0 < nimg; a0 += c->chunk) {
     const int nb = std::min(c->chunk, nimg - a0);
     if (inplane)
@@ -2547,7 +2580,8 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
         SPI_TRY(check_kernel("to_bf16_kernel"));
         c->count();
       }
-      SPI_TRY(launch_insert(c, c->slices.as<SliceDesc>() + (size_t)b0 * nsym, nvalid * nsym, g1));
+      SPI_TRY(launch_insert(c, c->slices.as<SliceDesc>() + (size_t)b0 * nsym, nvalid * nsym,
+                            insert_target(c, c->ngrids == 2 ? 1 : 0)));
       c->unfolded += nvalid;
       if (c->unfolded >= c->fold_every) SPI_TRY(fold_grids(c, false));
     }
@@ -2858,7 +2892,10 @@ static int bp_autotune_impl(spi_ctx* c, int force) {
   const size_t gbytes = grid_voxels(c) * sizeof(float4);
   for (int g = 0; g < c->ngrids; ++g) {
     SPI_CUDA(cudaMemsetAsync(c->gptr[g], 0, gbytes, c->stream));
-    if (c->accum) SPI_CUDA(cudaMemsetAsync(c->part[g].p, 0, gbytes, c->stream));
+    if (c->accum) {
+      SPI_CUDA(cudaMemsetAsync(c->part[g].p, 0, gbytes, c->stream));
+      c->part_zero[g] = true;
+    }
   }
   SPI_CUDA(cudaStreamSynchronize(c->stream));
   std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -3032,6 +3069,7 @@ int spi_bp_partial_add(spi_ctx* c, int g, const float* x_in, const float* w_in) 
   SPI_TRY(check_kernel("grid_add_kernel"));
   c->count();
   c->merged = true;
+  c->virgin = false;
   SPI_CUDA(cudaStreamSynchronize(c->stream));
   return 0;
 }

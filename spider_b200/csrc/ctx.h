@@ -46,6 +46,9 @@ struct spi_ctx {
   int fold_every = 0;                 // images between folds (compensated accumulation)
   long long unfolded = 0;             // images inserted into part[] since the last fold
   bool comp_dirty = false;            // comp[] may hold nonzero compensation terms
+  bool virgin = false;                // grids and comp[] are all zero and the grids are the library's own
+  bool part_zero[2] = {false, false}; // part[] / comp[] are known to be all zero
+  bool comp_zero[2] = {false, false};
   spi::DevBuf part[2];                // float4 partial sums of the images since the last fold
   spi::DevBuf comp[2];                // float4 low-order compensation of grid[] (two-sum error terms)
   float4* gptr[2] = {nullptr, nullptr};      // grids in use (owned or attached)
