@@ -1,0 +1,60 @@
+"""Reconstructions that reuse a context's grids: buffers kept over bp_close and
+same-size bp_open, partial grids exchanged with the grid by the first fold,
+grids left half done.  Each result equals a fresh context's to the order of
+the FP32 sums (2e-6)."""
+import numpy as np
+import pytest
+
+from spider_b200 import ops, synth
+
+pytestmark = pytest.mark.gpu
+NX, N = 24, 90
+
+
+@pytest.mark.parametrize("fold_every", [0, 16])
+@pytest.mark.parametrize("end", ["finish", "insert", "flush", "partial", "close"])
+def test_reconstruction_after_another(end, fold_every):
+    """The first reconstruction ends finished and closed, finished only, after an
+    insertion without a finish, flushed, or merged with a partial; with
+    one or two grids before and after; folds never, or within the images."""
+    rng = np.random.default_rng(7)
+    imgs = rng.standard_normal((2, N, NX, NX)).astype(np.float32)
+    ang = [synth.so3_angles(N, rng) for _ in range(2)]
+    half = synth.half_mask(N, rng)
+
+    def run(c, k, grids):
+        c.bp_open(NX, grids)
+        c.bp_insert(imgs[k][:50], ang[k][:50], half[:50] if grids == 2 else None)
+        c.bp_insert(imgs[k][50:], ang[k][50:], half[50:] if grids == 2 else None)
+        return c.bp_finish(("all", "1", "2") if grids == 2 else ("all",))
+
+    def fresh(k, grids):
+        c = ops.Context(0)
+        try:
+            c.set_accumulation(True, fold_every)
+            return run(c, k, grids)
+        finally:
+            c.close()
+    c = ops.Context(0)
+    try:
+        c.set_accumulation(True, fold_every)
+        for first, second in ((1, 1), (2, 1), (1, 2), (2, 2)):
+            if end in ("finish", "close"):
+                run(c, 0, first)
+                if end == "close":
+                    c.bp_close()
+            else:
+                c.bp_open(NX, first)
+                if end == "partial":
+                    x = rng.standard_normal((2 * NX, 2 * NX, NX + 1, 2)).astype(np.float32)
+                    c.bp_partial_add(x, np.ones(x.shape[:3], np.float32))
+                else:
+                    c.bp_insert(imgs[0], ang[0], half if first == 2 else None)
+                    if end == "flush":
+                        c.bp_flush()
+                        c.bp_insert(imgs[0][:20], ang[0][:20], half[:20] if first == 2 else None)
+            got, ref = run(c, 1, second), fresh(1, second)
+            for k, v in ref.items():
+                assert synth.rel_l2(got[k], v) <= 2e-6, (first, second, k)
+    finally:
+        c.close()
