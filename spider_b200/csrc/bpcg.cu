@@ -305,8 +305,28 @@ __global__ void absmax_kernel(const T* __restrict__ x, const CgRun* __restrict__
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(m));
 }
 
-// PRJCQ_N of projections kbase .. kbase+gridDim.x-1, accumulated in fixed
-// point in shared memory with native 32-bit integer atomics (exact and order
+// Layouts of the volume for the projector below: in[z][y][x] as
+// out[0][x][z][y] and out[1][x][y][z], by 32 x 32 tiles through shared memory.
+__global__ void __launch_bounds__(256) cg_layout_kernel(const double* __restrict__ in, int n, double* __restrict__ out) {
+  __shared__ double tile[32][33];
+  const size_t nn = (size_t)n * n;
+  const int which = blockIdx.z & 1, f = blockIdx.z >> 1;   // f: z (which 0) or y (which 1)
+  const int x0 = blockIdx.x * 32, t0 = blockIdx.y * 32;    // t: the other one
+  const size_t sf = which ? (size_t)n : nn, st = which ? nn : (size_t)n;
+  for (int i = threadIdx.y; i < 32; i += 8) {
+    const int t = t0 + i, x = x0 + threadIdx.x;
+    if (t < n && x < n) tile[i][threadIdx.x] = in[f * sf + t * st + x];
+  }
+  __syncthreads();
+  double* o = out + (size_t)which * nn * n;
+  for (int i = threadIdx.y; i < 32; i += 8) {
+    const int x = x0 + i, t = t0 + threadIdx.x;
+    if (t < n && x < n) o[x * nn + (size_t)f * n + t] = tile[threadIdx.x][i];
+  }
+}
+
+// PRJCQ_N of projections kbase, kbase + 1, .., accumulated in fixed point in
+// shared memory with native 32-bit integer atomics (exact and order
 // independent), written out as PROJT with the HIANG weights lb[k].
 //
 // Scale: every voxel whose projection can reach a pixel lies in a 2 x 2 x
@@ -320,146 +340,124 @@ __global__ void absmax_kernel(const T* __restrict__ x, const CgRun* __restrict__
 // pixel: the high sum stays within 0.95 * 2^31 + mcap, the low one within
 // mcap * 65535, and the pixel is hi * 65536 + lo exactly (a step of ~1e-11
 // max|x|).
-template <class T, bool WIDE, bool WT>
-__global__ void __launch_bounds__(512) prjcq_projt_kernel(const T* __restrict__ cube, const CgRun* __restrict__ runs,
-                                                          int nruns, const CgDM* __restrict__ dms,
-                                                          const int* __restrict__ lb, int kbase, int n, int ldp,
-                                                          const unsigned long long* __restrict__ maxabs_bits,
-                                                          float mcap, ProjtEntry<WT>* __restrict__ projt) {
+//
+// Bound: shared-memory wavefronts, eight atomics a voxel (WIDE).  A warp takes
+// 32 neighbouring voxel lines along y or z (`groups`, longest first) and walks
+// them together in x, each lane with the reference's sequential XB/YB steps
+// from the start of its own run, so every sample lands where the reference
+// puts it.  Of the two axes it takes the one along which the projected lines
+// are further apart, so that lanes seldom share a pixel; image rows are
+// `stride` words apart (1 or 31 mod 32) and are stored mirrored where the lines
+// run against that skew, so that neighbouring lanes fall into neighbouring
+// banks at any angle.  The volume is read from the layout in which the lanes'
+// voxels are contiguous (cg_layout_kernel).  At 128^3 with 1,000 directions 12.8 -> 3.9 us a projection against
+// one run a thread in run order (rows of n words, uncoalesced FP64 voxels).
+//
+// BAND (images too large for one CTA's shared memory): C CTAs per projection,
+// CTA b owning the pixel rows [b R, b R + R) (R = ceil(n / C)) and accumulating
+// rows [b R, b R + R + 2) of the fixed-point image, the two extra rows being
+// what its PROJT entries read beyond the band (I + N, and I + 1 wrapping to the
+// next row at the last column).  Lines that miss the band are skipped and the
+// others end once past it; integer sums make the tables identical to those of
+// one CTA.  (A 2-4 CTA cluster adding into one another's bands through
+// distributed shared memory was measured 3-8x slower at n = 256.)
+template <bool WIDE, bool WT, bool BAND>
+__global__ void __launch_bounds__(BAND ? 512 : 1024) prjcq_projt_kernel(
+    const double* __restrict__ layouts, const int2* __restrict__ lines, const int2* __restrict__ groups, int ngroups,
+    const CgDM* __restrict__ dms, const int* __restrict__ lb, int kbase, int n, int stride, int ldp, int C,
+    const unsigned long long* __restrict__ maxabs_bits, float mcap, ProjtEntry<WT>* __restrict__ projt) {
+  const int R = BAND ? (n + C - 1) / C : n;
+  const int proj = BAND ? blockIdx.x / C : blockIdx.x;
+  const int r0 = BAND ? (blockIdx.x % C) * R : 0;
+  const int r1 = min(n, r0 + R);                        // owned rows [r0, r1)
+  const int h1 = BAND ? min(n, r0 + R + 2) : n;         // accumulated rows [r0, h1)
+  const int words = (BAND ? R + 2 : n) * stride;        // per array
   extern __shared__ __align__(16) unsigned char smraw[];
-  int* hi = reinterpret_cast<int*>(smraw);
-  int* lo = hi + n * n;   // WIDE only
-  const int k = kbase + blockIdx.x;
-  for (int i = threadIdx.x; i < n * n * (WIDE ? 2 : 1); i += blockDim.x) hi[i] = 0;
-  const double maxabs = __longlong_as_double((long long)*maxabs_bits);
-  const double full = WIDE ? 0.95 * 140737488355328.0 : 0.95 * 2147483648.0;   // 2^47 or 2^31
-  const double scale = maxabs > 0.0 ? full / ((double)mcap * maxabs) : 0.0;
-  __syncthreads();
-  const CgDM dm = dms[k];
-  auto add = [&](int* p, double w) {
-    if (WIDE) {
-      const long long q = __double2ll_rn(w * scale);
-      atomicAdd(p, (int)(q >> 16));
-      atomicAdd(p + n * n, (int)(q & 0xffff));
-    } else {
-      atomicAdd(p, __double2int_rn(w * scale));
-    }
-  };
-  for (int ri = threadIdx.x; ri < nruns; ri += blockDim.x) {
-    const CgRun r = runs[ri];
-    const float fx = (float)(r.x - ldp), fy = (float)(r.y - ldp), fz = (float)(r.z - ldp);
-    float xb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, dm.d[0]), __fmul_rn(fy, dm.d[1])), __fmul_rn(fz, dm.d[2])), (float)ldp);
-    float yb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, dm.d[3]), __fmul_rn(fy, dm.d[4])), __fmul_rn(fz, dm.d[5])), (float)ldp);
-    T cnext = cube[(size_t)r.l1 - 1];   // the next voxel's value, loaded one step ahead
-    for (int j = r.l1; j <= r.l2; ++j) {
-      const T cv = cnext;
-      if (j < r.l2) cnext = cube[(size_t)j];
-      const int iqx = __float2int_rz(xb), iqy = __float2int_rz(yb);
-      if (iqx >= 1 && iqx < n && iqy >= 1 && iqy < n) {
-        const T dx = (T)__fsub_rn(xb, (float)iqx);
-        const T dy = rmul((T)__fsub_rn(yb, (float)iqy), cv);
-        const T dx1m = rsub((T)1, dx);
-        const T dy1m = rsub(cv, dy);
-        int* p = hi + (iqy - 1) * n + (iqx - 1);
-        add(p, (double)rmul(dx1m, dy1m));
-        add(p + 1, (double)rmul(dx, dy1m));
-        add(p + n, (double)rmul(dx1m, dy));
-        add(p + n + 1, (double)rmul(dx, dy));
-      }
-      xb = __fadd_rn(xb, dm.d[0]);
-      yb = __fadd_rn(yb, dm.d[3]);
-    }
-  }
-  __syncthreads();
-  const double inv = scale > 0.0 ? 1.0 / scale : 0.0;
-  const double w = lb ? (double)lb[k] : 1.0;
-  ProjtEntry<WT>* out = projt + (size_t)blockIdx.x * n * n;
-  auto val = [&](int i) {
-    return WIDE ? ((double)hi[i] * 65536.0 + (double)lo[i]) * inv : (double)hi[i] * inv;
-  };
-  for (int i = threadIdx.x; i < n * n; i += blockDim.x) projt_make<WT>(out + i, val, i + 1, n, w);
-}
-
-// The same projector for images too large for one CTA's shared memory: C
-// CTAs per projection, CTA b owning the pixel rows [b R, b R + R) (R =
-// ceil(n / C)) and accumulating rows [b R, b R + R + 2) of the fixed-point
-// image, the two extra rows being what its PROJT entries read beyond the
-// band (I + N, and I + 1 wrapping to the next row at the last column).  Every
-// CTA walks all runs with the reference's sequential XB/YB steps and splats
-// only into its rows, so all atomics stay in its own shared memory; the
-// voxels of other bands cost four instructions each.  Integer sums make the
-// tables identical to those of the one-CTA kernel.  (A 2-4 CTA cluster
-// adding into one another's bands through distributed shared memory was
-// measured 3-8x slower at n = 256.)
-template <class T, bool WIDE, bool WT>
-__global__ void __launch_bounds__(512) prjcq_projt_band_kernel(
-    const T* __restrict__ cube, const CgRun* __restrict__ runs, int nruns, const CgDM* __restrict__ dms,
-    const int* __restrict__ lb, int kbase, int n, int ldp, int C, const unsigned long long* __restrict__ maxabs_bits,
-    float mcap, ProjtEntry<WT>* __restrict__ projt) {
-  const int R = (n + C - 1) / C;
-  const int proj = blockIdx.x / C, b = blockIdx.x % C;
-  const int r0 = b * R;
-  const int r1 = min(n, r0 + R);             // owned rows [r0, r1)
-  const int h1 = min(n, r0 + R + 2);         // accumulated rows [r0, h1)
-  const int words = (R + 2) * n;             // per array
-  extern __shared__ __align__(16) unsigned char smraw[];
-  int* hi = reinterpret_cast<int*>(smraw);   // lo = hi + words (WIDE)
+  int* hi = reinterpret_cast<int*>(smraw);              // lo = hi + words (WIDE)
   const int k = kbase + proj;
   for (int i = threadIdx.x; i < words * (WIDE ? 2 : 1); i += blockDim.x) hi[i] = 0;
   const double maxabs = __longlong_as_double((long long)*maxabs_bits);
   const double full = WIDE ? 0.95 * 140737488355328.0 : 0.95 * 2147483648.0;   // 2^47 or 2^31
   const double scale = maxabs > 0.0 ? full / ((double)mcap * maxabs) : 0.0;
   __syncthreads();
-  auto add = [&](int local, double w) {
+  auto add = [&](int* p, double w) {
     if (WIDE) {
-      const long long q = __double2ll_rn(w * scale);
-      atomicAdd(hi + local, (int)(q >> 16));
-      atomicAdd(hi + words + local, (int)(q & 0xffff));
+      // q = w * scale rounded to an integer (|q| < 2^51) by adding 1.5 * 2^52:
+      // the sum's low 51 bits are q's, and those of the addend are zero
+      const long long q = __double_as_longlong(__dadd_rn(__dmul_rn(w, scale), 6755399441055744.0));
+      atomicAdd(p, (int)(q >> 16));
+      atomicAdd(p + words, (int)(q & 0xffff));
     } else {
-      atomicAdd(hi + local, __double2int_rn(w * scale));
+      atomicAdd(p, __double2int_rn(w * scale));
     }
   };
   const CgDM dm = dms[k];
-  const float ystep = dm.d[3];
-  for (int ri = threadIdx.x; ri < nruns; ri += blockDim.x) {
-    const CgRun r = runs[ri];
-    const float fx = (float)(r.x - ldp), fy = (float)(r.y - ldp), fz = (float)(r.z - ldp);
+  const bool along_y = fabsf(dm.d[1]) + fabsf(dm.d[4]) >= fabsf(dm.d[2]) + fabsf(dm.d[5]);
+  const float ax = along_y ? dm.d[1] : dm.d[2], ay = along_y ? dm.d[4] : dm.d[5];
+  const bool mirror = ((ax < 0.0f) != (ay < 0.0f)) != ((stride & 31) == 31);
+  const int step = mirror ? -1 : 1;
+  int* const origin = hi + (mirror ? n - 1 : 0);
+  const size_t nn = (size_t)n * n;
+  const double* const vol = layouts + (along_y ? 0 : nn * n);
+  const int lane = threadIdx.x & 31;
+  for (int g = threadIdx.x >> 5; g < ngroups; g += blockDim.x >> 5) {
+    const int2 G = groups[g];
+    const int t = min(G.y + lane, n - 1);
+    int2 run = lines[G.x * n + t];
+    if (G.y + lane >= n) run.y = 0;
+    const float fx = (float)(run.x + 1 - ldp);
+    const float fy = (float)((along_y ? t : G.x) + 1 - ldp), fz = (float)((along_y ? G.x : t) + 1 - ldp);
     float xb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, dm.d[0]), __fmul_rn(fy, dm.d[1])), __fmul_rn(fz, dm.d[2])), (float)ldp);
     float yb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, dm.d[3]), __fmul_rn(fy, dm.d[4])), __fmul_rn(fz, dm.d[5])), (float)ldp);
-    // A run whose rows all miss the band is skipped: its YB is linear in the
-    // step up to the walk's rounding (well under the 2-row margin).
-    const float ye = yb + (float)(r.l2 - r.l1) * ystep;
-    if (fmaxf(yb, ye) + 2.0f < (float)r0 || fminf(yb, ye) - 2.0f > (float)(h1 + 1)) continue;
-    for (int j = r.l1; j <= r.l2; ++j) {
-      const int iqy = __float2int_rz(yb);
-      // rows iqy-1 and iqy (0-based) of the splat; skip unless one is accumulated here
-      if (iqy >= r0 && iqy - 1 < h1) {
-        const int iqx = __float2int_rz(xb);
-        if (iqx >= 1 && iqx < n && iqy >= 1 && iqy < n) {
-          const T cv = cube[(size_t)j - 1];
-          const T dx = (T)__fsub_rn(xb, (float)iqx);
-          const T dy = rmul((T)__fsub_rn(yb, (float)iqy), cv);
-          const T dx1m = rsub((T)1, dx);
-          const T dy1m = rsub(cv, dy);
-          const int ya = iqy - 1, yb1 = iqy;   // pixel rows, 0-based
-          if (ya >= r0 && ya < h1) {
-            const int l = (ya - r0) * n + (iqx - 1);
-            add(l, (double)rmul(dx1m, dy1m));
-            add(l + 1, (double)rmul(dx, dy1m));
-          }
-          if (yb1 >= r0 && yb1 < h1) {
-            const int l = (yb1 - r0) * n + (iqx - 1);
-            add(l, (double)rmul(dx1m, dy));
-            add(l + 1, (double)rmul(dx, dy));
-          }
+    if (BAND) {
+      // YB is linear in the step up to the walk's rounding, well under the
+      // margin of 2 rows
+      const float ystep = dm.d[3];
+      const float ye = yb + (float)(run.y - 1) * ystep;
+      if (fmaxf(yb, ye) + 2.0f < (float)r0 || fminf(yb, ye) - 2.0f > (float)(h1 + 1)) run.y = 0;
+      if (ystep != 0.0f) {
+        const float past = ((ystep > 0.0f ? (float)(h1 + 3) : (float)(r0 - 3)) - yb) / ystep;
+        run.y = min(run.y, (int)fminf(fmaxf(past, 0.0f), 65536.0f) + 1);
+      }
+    }
+    const int first = __reduce_min_sync(0xffffffffu, run.y > 0 ? run.x : n);
+    const int last = __reduce_max_sync(0xffffffffu, run.y > 0 ? run.x + run.y : 0);
+    const double* src = vol + (size_t)G.x * n + t;
+    auto voxel = [&](int x, double loaded) {
+      if ((unsigned)(x - run.x) >= (unsigned)run.y) return;
+      const int iqx = __float2int_rz(xb), iqy = __float2int_rz(yb);
+      const bool here = !BAND || (iqy >= r0 && iqy - 1 < h1);
+      if (here && iqx >= 1 && iqx < n && iqy >= 1 && iqy < n) {
+        double cv = BAND ? __ldg(src + x * nn) : loaded;
+        // infinities (scale 0) and NaN add nothing, in WIDE as by conversion
+        if (WIDE && !(fabs(cv) <= 1.7976931348623157e308)) cv = 0.0;
+        const double dx = (double)__fsub_rn(xb, (float)iqx);
+        const double dy = rmul((double)__fsub_rn(yb, (float)iqy), cv);
+        const double dx1m = rsub(1.0, dx);
+        const double dy1m = rsub(cv, dy);
+        int* p = origin + (iqy - 1 - r0) * stride + (mirror ? 1 - iqx : iqx - 1);
+        if (!BAND || iqy - 1 >= r0) {   // iqy - 1 < h1 holds
+          add(p, rmul(dx1m, dy1m));
+          add(p + step, rmul(dx, dy1m));
         }
-      } else if ((ystep > 0.0f && iqy > h1) || (ystep < 0.0f && iqy < r0)) {
-        // past the band: adding DM(4) of one sign moves YB (and its
-        // truncation) one way only, so no later voxel of the run reaches it
-        break;
+        if (!BAND || iqy < h1) {        // iqy >= r0 holds
+          add(p + stride, rmul(dx1m, dy));
+          add(p + stride + step, rmul(dx, dy));
+        }
       }
       xb = __fadd_rn(xb, dm.d[0]);
       yb = __fadd_rn(yb, dm.d[3]);
+    };
+    if (BAND) {
+      for (int x = first; x < last; ++x) voxel(x, 0.0);
+    } else {
+      for (int x = first; x < last; x += 4) {
+        double c[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) c[u] = __ldg(src + min(x + u, n - 1) * nn);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) voxel(x + u, c[u]);
+      }
     }
   }
   __syncthreads();
@@ -467,8 +465,9 @@ __global__ void __launch_bounds__(512) prjcq_projt_band_kernel(
   const double w = lb ? (double)lb[k] : 1.0;
   ProjtEntry<WT>* out = projt + (size_t)proj * n * n;
   auto val = [&](int pix) {
-    const int l = pix - r0 * n;
-    return WIDE ? ((double)hi[l] * 65536.0 + (double)hi[words + l]) * inv : (double)hi[l] * inv;
+    const int row = pix / n, col = pix - row * n;
+    const int* p = origin + (row - r0) * stride + step * col;
+    return WIDE ? ((double)p[0] * 65536.0 + (double)p[words]) * inv : (double)p[0] * inv;
   };
   for (int i = r0 * n + threadIdx.x; i < r1 * n; i += blockDim.x) projt_make<WT>(out + i, val, i + 1, n, w);
 }
@@ -703,6 +702,7 @@ struct CgProblem {
   float ri;
   std::vector<CgRun> runs;
   long long nvox = 0;
+  int ngroups = 0;   // projector groups (cg_lines)
 };
 
 static int cg_setup(spi_ctx* c, int n, float ri, CgProblem& pb) {
@@ -821,6 +821,15 @@ static int mixed_bands(int n, bool wide) {
   }
   return C;
 }
+// Words between rows of the fixed-point image: the next number from n up that
+// is 1 or 31 mod 32.  With the extra words the largest images of a form still
+// fit the 227 KB of a CTA: 160 rows of 161 in 64 bits, 226 of 255 in 32, and
+// 58 of 447 in 64 bits (n = 443 in 8 bands).
+static constexpr int kProjSmem = 227 * 1024;
+static int proj_stride(int n) {
+  while ((n & 31) != 1 && (n & 31) != 31) ++n;
+  return n;
+}
 static bool mixed_fits(int n, bool wide) { return mixed_bands(n, wide) > 0; }
 
 // A^T from PROJT tables of images [k0, k1), 64 images per launch
@@ -838,16 +847,45 @@ static int launch_backproject_projt(spi_ctx* c, const CgProblem& pb, T* cube, co
   return 0;
 }
 
+// Tables of the projector of the mixed modes: cg_buf[8] = the run {first x,
+// voxels} of each line [n][n], then the groups {f, t} of 32 lines t .. t+31 at
+// the other coordinate f, longest first; cg_buf[9] = room for the two layouts.
+// The table is the same for (y, z) and (z, y): PREPCUB_S compares sums of
+// squared integers, which are exact.
+static int cg_lines(spi_ctx* c, CgProblem& pb) {
+  const int n = pb.n;
+  std::vector<int2> tab((size_t)n * n, make_int2(0, 0));
+  std::vector<int> lo(n, n), hi(n, -1);
+  for (const CgRun& r : pb.runs) {
+    tab[(size_t)(r.z - 1) * n + (r.y - 1)] = make_int2(r.x - 1, r.l2 - r.l1 + 1);
+    lo[r.z - 1] = std::min(lo[r.z - 1], r.y - 1);
+    hi[r.z - 1] = std::max(hi[r.z - 1], r.y - 1);
+  }
+  std::vector<std::pair<int, int2>> gs;
+  for (int f = 0; f < n; ++f)
+    for (int t = lo[f]; t <= hi[f]; t += 32) {
+      int len = 0;
+      for (int u = t; u < std::min(n, t + 32); ++u) len = std::max(len, tab[(size_t)f * n + u].y);
+      gs.push_back({len, make_int2(f, t)});
+    }
+  std::stable_sort(gs.begin(), gs.end(), [](auto& a, auto& b) { return a.first > b.first; });
+  pb.ngroups = (int)gs.size();
+  for (auto& g : gs) tab.push_back(g.second);
+  SPI_TRY(c->cg_buf[8].ensure(tab.size() * sizeof(int2)));
+  SPI_TRY(c->cg_buf[9].ensure(2 * (size_t)n * n * n * sizeof(double)));
+  SPI_CUDA(cudaMemcpyAsync(c->cg_buf[8].p, tab.data(), tab.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
+  return 0;
+}
+
 // A then A^T (BCKE += A^T A BCKP) chunk by chunk through PROJT tables
-template <class T, bool WIDE, bool WT>
-static int launch_normal_projt(spi_ctx* c, const CgProblem& pb, const T* x, T* out, const CgDM* dms, const int* lb,
+template <bool WIDE, bool WT>
+static int launch_normal_projt(spi_ctx* c, const CgProblem& pb, const double* x, double* out, const CgDM* dms, const int* lb,
                                int nang, ProjtEntry<WT>* projt, unsigned long long* maxabs) {
   const int n = pb.n;
   const int K = projt_chunk(n, nang, sizeof(ProjtEntry<WT>));
-  const size_t smem = (size_t)n * n * (WIDE ? 8 : 4);
   // fixed-point scale of the projector: max |x| over the sphere
   SPI_CUDA(cudaMemsetAsync(maxabs, 0, sizeof(unsigned long long), c->stream));
-  absmax_kernel<T><<<blocks_for(c, pb.nvox, 256), 256, 0, c->stream>>>(x, c->cg_buf[0].as<CgRun>(), c->cg_buf[1].as<int>(),
+  absmax_kernel<double><<<blocks_for(c, pb.nvox, 256), 256, 0, c->stream>>>(x, c->cg_buf[0].as<CgRun>(), c->cg_buf[1].as<int>(),
                                                                       c->cg_buf[2].as<int>(), pb.nvox, maxabs);
   SPI_TRY(check_kernel("absmax_kernel"));
   c->count();
@@ -856,23 +894,31 @@ static int launch_normal_projt(spi_ctx* c, const CgProblem& pb, const T* x, T* o
   static std::atomic<unsigned long long> attr_set{0};
   const unsigned long long bit = 1ull << (c->device & 63);
   if (!(attr_set.load() & bit)) {
-    cudaFuncSetAttribute(prjcq_projt_kernel<T, WIDE, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(prjcq_projt_band_kernel<T, WIDE, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    cudaFuncSetAttribute(prjcq_projt_kernel<WIDE, WT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kProjSmem);
+    cudaFuncSetAttribute(prjcq_projt_kernel<WIDE, WT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kProjSmem);
     attr_set.fetch_or(bit);
   }
   const int C = mixed_bands(n, WIDE);
   if (C < 1) return fail(kInvalid, "BP CG: n = %d too large for the mixed precision modes", n);
+  const int stride = proj_stride(n);
+  const size_t smem = (size_t)(C == 1 ? n : (n + C - 1) / C + 2) * stride * (WIDE ? 8 : 4);
+  double* const layouts = c->cg_buf[9].as<double>();
+  const int2* const lines = c->cg_buf[8].as<int2>();
+  cg_layout_kernel<<<dim3((n + 31) / 32, (n + 31) / 32, 2 * n), dim3(32, 8), 0, c->stream>>>(x, n, layouts);
+  SPI_TRY(check_kernel("cg_layout_kernel"));
+  c->count();
   for (int k0 = 0; k0 < nang; k0 += K) {
     const int kc = std::min(K, nang - k0);
-    if (C == 1)
-      prjcq_projt_kernel<T, WIDE, WT><<<kc, 512, smem, c->stream>>>(x, c->cg_buf[0].as<CgRun>(), (int)pb.runs.size(), dms,
-                                                                 lb, k0, n, pb.ldp, maxabs, mcap, projt);
-    else
-      prjcq_projt_band_kernel<T, WIDE, WT><<<kc * C, 512, band_bytes(n, C, WIDE), c->stream>>>(
-          x, c->cg_buf[0].as<CgRun>(), (int)pb.runs.size(), dms, lb, k0, n, pb.ldp, C, maxabs, mcap, projt);
+    auto launch = [&](auto kern, int threads) {
+      kern<<<kc * C, threads, smem, c->stream>>>(layouts, lines, lines + (size_t)n * n, pb.ngroups, dms, lb, k0, n,
+                                                 stride, pb.ldp, C, maxabs, mcap, projt);
+    };
+    // one CTA per SM above half of its shared memory: twice the warps then
+    if (C == 1) launch(prjcq_projt_kernel<WIDE, WT, false>, smem > kProjSmem / 2 ? 1024 : 512);
+    else launch(prjcq_projt_kernel<WIDE, WT, true>, 512);
     SPI_TRY(check_kernel("prjcq_projt_kernel"));
     c->count();
-    SPI_TRY((launch_backproject_projt<T, WT>(c, pb, out, projt, dms, k0, k0, k0 + kc)));
+    SPI_TRY((launch_backproject_projt<double, WT>(c, pb, out, projt, dms, k0, k0, k0 + kc)));
   }
   return 0;
 }
@@ -1353,6 +1399,7 @@ static int bpcg_run(spi_ctx* c, const float* projs, int n, int nang, const float
     SPI_TRY(c->cg_buf[5].ensure((size_t)pj_rows * n * n * sizeof(T) +
                                 (sizeof(T) != sizeof(float) ? pcount * sizeof(float) : 0) + 4));
   SPI_TRY(c->cg_buf[6].ensure(3 * vb));
+  if (mixed) SPI_TRY(cg_lines(c, pb));
   SPI_TRY(c->cg_buf[7].ensure(sizeof(CgScal) + 64 + (size_t)nang * sizeof(int)));
   T* cb = c->cg_buf[4].as<T>();
   T* pj = c->cg_buf[5].as<T>();
@@ -1474,15 +1521,17 @@ static int bpcg_run(spi_ctx* c, const float* projs, int n, int nang, const float
       SPI_TRY((fbs_normal<T, T>(c, pb, fs, bckp, bcke, dlb, kb, ke, c->cg_buf[3].as<CgDM>())));
     } else if (mixed) {
       auto* mx = reinterpret_cast<unsigned long long*>(acc + 7);
-      if (wide && wtab)
-        SPI_TRY((launch_normal_projt<T, true, true>(c, pb, bckp, bcke, mdm, mlb, mc,
-                                                    static_cast<ProjtEntry<true>*>(projt), mx)));
-      else if (wide)
-        SPI_TRY((launch_normal_projt<T, true, false>(c, pb, bckp, bcke, mdm, mlb, mc,
+      if constexpr (sizeof(T) == 8) {   // `mixed` holds for FP64 vectors only
+        if (wide && wtab)
+          SPI_TRY((launch_normal_projt<true, true>(c, pb, bckp, bcke, mdm, mlb, mc,
+                                                   static_cast<ProjtEntry<true>*>(projt), mx)));
+        else if (wide)
+          SPI_TRY((launch_normal_projt<true, false>(c, pb, bckp, bcke, mdm, mlb, mc,
+                                                    static_cast<ProjtEntry<false>*>(projt), mx)));
+        else
+          SPI_TRY((launch_normal_projt<false, false>(c, pb, bckp, bcke, mdm, mlb, mc,
                                                      static_cast<ProjtEntry<false>*>(projt), mx)));
-      else
-        SPI_TRY((launch_normal_projt<T, false, false>(c, pb, bckp, bcke, mdm, mlb, mc,
-                                                      static_cast<ProjtEntry<false>*>(projt), mx)));
+      }
     } else {
       SPI_TRY(launch_project<T>(c, pb, bckp, mdm, mc, pj));
       SPI_TRY(launch_backproject<T>(c, pb, bcke, pj, mdm, mlb, mc));

@@ -86,7 +86,7 @@ struct spi_ctx {
   int pjf_n = 0;                      // cube size of those plans
   spi::DevBuf pj_v4;                  // PJ 3Q: the volume as float4 quads of x/y neighbours
   spi::DevBuf pj_rows;                // PJ 3Q forward: runs in (y, |z|) order, then the row tasks
-  spi::DevBuf cg_buf[8];
+  spi::DevBuf cg_buf[10];
   spi::DevBuf cg_fbs[4];              // FBS: 3D scratch + table, 2D chunk scratch, segments, DM(1..9)
   spi::HostBuf hbuf;
 
