@@ -472,35 +472,77 @@ __global__ void __launch_bounds__(BAND ? 512 : 1024) prjcq_projt_kernel(
   for (int i = r0 * n + threadIdx.x; i < r1 * n; i += blockDim.x) projt_make<WT>(out + i, val, i + 1, n, w);
 }
 
-// BCKPJ_LIN from PROJT tables of images [k0, k1) (table of image k at
-// projt + (k - kbase) * n * n), accumulating in T.
+// A float in {0} or [2^-126, 2^127] as a double by integer arithmetic: the
+// converter runs at a quarter of the rate and has the four terms to widen.
+__device__ __forceinline__ double widen_nonneg(float f) {
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double(b ? (int)((b >> 3) + 0x38000000u) : 0, (int)(b << 29));
+}
+
+// BCKPJ_LIN from PROJT tables of images [k0, k1), k1 - k0 <= 64 (table of
+// image k at projt + (k - kbase) * n * n), accumulating in T, one thread a
+// voxel, the images in order.
+//
+// Bound: instruction issue and the converter unit.  `perm` lists the sphere's
+// voxels by 8 x 4 x 4 boxes, so that the table entries of a warp, and of the
+// warps of a block, lie together; the transforms come from shared memory, and
+// four entries are asked for before the first is used.  PREPCUB_S keeps RI +
+// MODE + 1 <= N/2 (a larger radius is refused before any result), so positions
+// lie in [2, N - 1] and truncation is rounding down, which adding 2^23 does.
+// At 128^3 3.4 -> 2.05 us an image against voxels in run order, transforms
+// from global memory and all conversions through the converter.
 template <class T, bool WIDE>
-__global__ void __launch_bounds__(256) bckpj_projt_kernel(T* __restrict__ cube, const CgRun* __restrict__ runs,
-                                                          const int* __restrict__ vox_run, const int* __restrict__ vox_off,
-                                                          long long nvox, const ProjtEntry<WIDE>* __restrict__ projt,
+__global__ void __launch_bounds__(256) bckpj_projt_kernel(T* __restrict__ cube, const int2* __restrict__ lines,
+                                                          const int* __restrict__ perm, int nvox,
+                                                          const ProjtEntry<WIDE>* __restrict__ projt,
                                                           const CgDM* __restrict__ dms, int kbase, int k0, int k1, int n,
                                                           int ldp) {
-  for (long long v = blockIdx.x * (long long)blockDim.x + threadIdx.x; v < nvox; v += (long long)gridDim.x * blockDim.x) {
-    const CgRun r = runs[vox_run[v]];
-    const int jt = vox_off[v];
-    const size_t lin = (size_t)r.l1 - 1 + jt;
-    T c = cube[lin];
-    const float fx = (float)(r.x - ldp), fy = (float)(r.y - ldp), fz = (float)(r.z - ldp), fj = (float)jt;
-    for (int k = k0; k < k1; ++k) {
-      const CgDM dm = dms[k];
-      const float xb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, dm.d[0]), __fmul_rn(fy, dm.d[1])), __fmul_rn(fz, dm.d[2])), (float)ldp);
-      const float yb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, dm.d[3]), __fmul_rn(fy, dm.d[4])), __fmul_rn(fz, dm.d[5])), (float)ldp);
-      const float xbb = __fadd_rn(xb, __fmul_rn(fj, dm.d[0]));
-      const float ybb = __fadd_rn(yb, __fmul_rn(fj, dm.d[3]));
-      const int iqx = __float2int_rz(xbb), iqy = __float2int_rz(ybb);
-      const int I = (iqy - 1) * n + iqx;  // PROJT column, 1-based
-      double b1 = 0.0, b2 = 0.0, b3 = 0.0, b4 = 0.0;
-      if (I >= 1 && I <= n * n - n - 1) projt_load(projt + (size_t)(k - kbase) * n * n + (I - 1), b1, b2, b3, b4);
-      const T dy = (T)__fsub_rn(ybb, (float)iqy), dx = (T)__fsub_rn(xbb, (float)iqx);
-      c = radd(radd(radd(c, (T)b1), rmul(dy, (T)b2)), rmul(dx, radd((T)b3, rmul(dy, (T)b4))));
-    }
-    cube[lin] = c;
+  __shared__ float4 sx[64], sy[64];   // {DM1, DM2, DM3, -}, {DM4, DM5, DM6, -}
+  if (threadIdx.x < k1 - k0) {
+    const CgDM dm = dms[k0 + threadIdx.x];
+    sx[threadIdx.x] = make_float4(dm.d[0], dm.d[1], dm.d[2], 0.0f);
+    sy[threadIdx.x] = make_float4(dm.d[3], dm.d[4], dm.d[5], 0.0f);
   }
+  __syncthreads();
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= nvox) return;
+  const int lin = perm[v];
+  const int line = lin / n;
+  const int2 run = lines[line];
+  T c = cube[lin];
+  const float fx = (float)(run.x + 1 - ldp), fy = (float)(line % n + 1 - ldp), fz = (float)(line / n + 1 - ldp);
+  const float fj = (float)(lin - line * n - run.x), fl = (float)ldp;
+  const int limit = n * n - n - 1;
+  const ProjtEntry<WIDE>* table = projt + (size_t)(k0 - kbase) * n * n - 1;
+  for (int k = 0; k < k1 - k0; k += 4) {
+    double b[4][4];
+    float dx[4], dy[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float4 mx = sx[min(k + u, 63)], my = sy[min(k + u, 63)];
+      // XB = ((X-LDP)*DM1 + (Y-LDP)*DM2 + (Z-LDP)*DM3) + LDPNM ; XBB = XB + JT*DM1
+      const float xb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, mx.x), __fmul_rn(fy, mx.y)), __fmul_rn(fz, mx.z)), fl);
+      const float yb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, my.x), __fmul_rn(fy, my.y)), __fmul_rn(fz, my.z)), fl);
+      const float xbb = __fadd_rn(xb, __fmul_rn(fj, mx.x));
+      const float ybb = __fadd_rn(yb, __fmul_rn(fj, my.x));
+      const float tx = __fadd_rd(xbb, 8388608.0f), ty = __fadd_rd(ybb, 8388608.0f);
+      const int iqx = __float_as_int(tx) & 0x7fffff, iqy = __float_as_int(ty) & 0x7fffff;
+      dx[u] = __fsub_rn(xbb, __fsub_rn(tx, 8388608.0f));
+      dy[u] = __fsub_rn(ybb, __fsub_rn(ty, 8388608.0f));
+      const int I = (iqy - 1) * n + iqx;  // PROJT column, 1-based
+      b[u][0] = b[u][1] = b[u][2] = b[u][3] = 0.0;
+      if (k + u < k1 - k0 && I >= 1 && I <= limit)
+        projt_load(table + (size_t)(k + u) * n * n + I, b[u][0], b[u][1], b[u][2], b[u][3]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (k + u < k1 - k0) {
+        const T ex = (T)widen_nonneg(dx[u]), ey = (T)widen_nonneg(dy[u]);
+        c = radd(radd(radd(c, (T)b[u][0]), rmul(ey, (T)b[u][1])), rmul(ex, radd((T)b[u][2], rmul(ey, (T)b[u][3]))));
+      }
+    }
+  }
+  cube[lin] = c;
 }
 
 // Same splat with global atomics, for images that exceed shared memory.
@@ -702,7 +744,8 @@ struct CgProblem {
   float ri;
   std::vector<CgRun> runs;
   long long nvox = 0;
-  int ngroups = 0;   // projector groups (cg_lines)
+  int ngroups = 0;   // projector groups, and where the voxel order starts (cg_lines)
+  size_t perm = 0;
 };
 
 static int cg_setup(spi_ctx* c, int n, float ri, CgProblem& pb) {
@@ -838,18 +881,42 @@ static int launch_backproject_projt(spi_ctx* c, const CgProblem& pb, T* cube, co
                                     const CgDM* dms, int kbase, int k0, int k1) {
   for (int a = k0; a < k1; a += 64) {
     const int b = std::min(k1, a + 64);
-    bckpj_projt_kernel<T, WIDE><<<blocks_for(c, pb.nvox, 256), 256, 0, c->stream>>>(
-        cube, c->cg_buf[0].as<CgRun>(), c->cg_buf[1].as<int>(), c->cg_buf[2].as<int>(), pb.nvox, projt, dms, kbase, a,
-        b, pb.n, pb.ldp);
+    if (pb.nvox == 0) break;
+    bckpj_projt_kernel<T, WIDE><<<(unsigned)((pb.nvox + 255) / 256), 256, 0, c->stream>>>(
+        cube, c->cg_buf[8].as<int2>(), reinterpret_cast<const int*>(c->cg_buf[8].as<int2>() + pb.perm), (int)pb.nvox,
+        projt, dms, kbase, a, b, pb.n, pb.ldp);
     SPI_TRY(check_kernel("bckpj_projt_kernel"));
     c->count();
   }
   return 0;
 }
 
+// The sphere's voxels of 8 x 4 x 4 boxes, one warp a box and one lane a line
+__global__ void __launch_bounds__(256) cg_perm_kernel(const int2* __restrict__ lines, const int* __restrict__ start, int n,
+                                                      int bx, int by, int nbox, int* __restrict__ perm) {
+  const int box = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (box >= nbox) return;
+  const int x = box % bx * 8, y = box / bx % by * 4 + (lane & 3), z = box / bx / by * 4 + (lane >> 2);
+  int a = 0, e = 0;
+  if (lane < 16 && y < n && z < n) {
+    const int2 run = lines[z * n + y];
+    a = max(x, run.x);
+    e = min(x + 8, run.x + run.y);
+  }
+  const int cnt = max(e - a, 0);
+  int before = cnt;
+  for (int o = 1; o < 16; o <<= 1) {
+    const int w = __shfl_up_sync(0xffffffffu, before, o);
+    if (lane >= o) before += w;
+  }
+  int* out = perm + start[box] + before - cnt;
+  for (int i = 0; i < cnt; ++i) out[i] = (z * n + y) * n + a + i;
+}
+
 // Tables of the projector of the mixed modes: cg_buf[8] = the run {first x,
 // voxels} of each line [n][n], then the groups {f, t} of 32 lines t .. t+31 at
-// the other coordinate f, longest first; cg_buf[9] = room for the two layouts.
+// the other coordinate f, longest first, then the sphere's voxels by 8 x 4 x 4
+// boxes (0-based linear indices); cg_buf[9] = room for the two layouts.
 // The table is the same for (y, z) and (z, y): PREPCUB_S compares sums of
 // squared integers, which are exact.
 static int cg_lines(spi_ctx* c, CgProblem& pb) {
@@ -871,9 +938,24 @@ static int cg_lines(spi_ctx* c, CgProblem& pb) {
   std::stable_sort(gs.begin(), gs.end(), [](auto& a, auto& b) { return a.first > b.first; });
   pb.ngroups = (int)gs.size();
   for (auto& g : gs) tab.push_back(g.second);
-  SPI_TRY(c->cg_buf[8].ensure(tab.size() * sizeof(int2)));
+  // where the voxels of each 8 x 4 x 4 box (x fastest) start in the order
+  const int bx = (n + 7) / 8, by = (n + 3) / 4, nbox = bx * by * by;
+  std::vector<int> start((size_t)nbox + 2, 0);
+  for (const CgRun& r : pb.runs)
+    for (int x = r.x - 1, e = r.x + r.l2 - r.l1; x < e; x = (x / 8 + 1) * 8)
+      start[((r.z - 1) / 4 * by + (r.y - 1) / 4) * bx + x / 8 + 1] += std::min(e, (x / 8 + 1) * 8) - x;
+  for (int i = 0; i < nbox; ++i) start[i + 1] += start[i];
+  const size_t box0 = tab.size();
+  for (int i = 0; i < (nbox + 1) / 2; ++i) tab.push_back(make_int2(start[2 * i], start[2 * i + 1]));
+  pb.perm = tab.size();
+  SPI_TRY(c->cg_buf[8].ensure(tab.size() * sizeof(int2) + (size_t)std::max(pb.nvox, 1ll) * sizeof(int)));
   SPI_TRY(c->cg_buf[9].ensure(2 * (size_t)n * n * n * sizeof(double)));
   SPI_CUDA(cudaMemcpyAsync(c->cg_buf[8].p, tab.data(), tab.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
+  const int2* d = c->cg_buf[8].as<int2>();
+  cg_perm_kernel<<<(nbox + 7) / 8, 256, 0, c->stream>>>(d, reinterpret_cast<const int*>(d + box0), n, bx, by, nbox,
+                                                        reinterpret_cast<int*>(c->cg_buf[8].as<int2>() + pb.perm));
+  SPI_TRY(check_kernel("cg_perm_kernel"));
+  c->count();
   return 0;
 }
 

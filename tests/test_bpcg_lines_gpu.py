@@ -1,4 +1,5 @@
-"""The mixed-precision BP CG operators (lines of 32 walked together) against the FP64 operators, at box sizes around their
+"""The mixed-precision BP CG operators (lines of 32 walked together, voxels in
+8 x 4 x 4 boxes) against the FP64 operators, at box sizes around their
 granules and at view directions along the axes and diagonals, where lines of
 a warp project onto one another or onto one image row or column.
 
