@@ -37,8 +37,9 @@ struct CgDM {
 };
 
 static void prepcub_s(int n, float ri, int ldp, std::vector<CgRun>& runs) {
+  // RC = t3^2 + (t2^2 + t^2) grows with |t3|, so a line's run is the voxels up
+  // to the last step h from the centre with RC <= r, cut at the box
   const float r = ri * ri;
-  int nmat = 0;
   runs.clear();
   for (int i1 = 1; i1 <= n; ++i1) {
     float t = (float)(i1 - ldp);
@@ -46,20 +47,28 @@ static void prepcub_s(int n, float ri, int ldp, std::vector<CgRun>& runs) {
     for (int i2 = 1; i2 <= n; ++i2) {
       float t2 = (float)(i2 - ldp);
       float yy = t2 * t2 + xx;
-      bool first = true;
-      for (int i3 = 1; i3 <= n; ++i3) {
-        ++nmat;
-        float t3 = (float)(i3 - ldp);
-        float rc = t3 * t3 + yy;
-        if (first) {
-          if (rc > r) continue;
-          first = false;
-          runs.push_back(CgRun{nmat, nmat, i3, i2, i1});
-        } else if (rc <= r) {
-          runs.back().l2 = nmat;
-        }
-      }
+      if (yy > r) continue;
+      int h = (int)std::min((float)n, std::sqrt(r - yy));
+      while (h < n && (float)(h + 1) * (float)(h + 1) + yy <= r) ++h;
+      while (h > 0 && !((float)h * (float)h + yy <= r)) --h;
+      int a = std::max(1, ldp - h), e = std::min(n, ldp + h);
+      if (r != r) a = e = 1;   // no comparison holds
+      const int line = ((i1 - 1) * n + (i2 - 1)) * n;
+      runs.push_back(CgRun{line + a, line + e, a, i2, i1});
     }
+  }
+}
+
+// run and offset in the run of every sphere voxel; one warp a run, whose first
+// voxel is number start[run]
+__global__ void __launch_bounds__(256) cg_voxels_kernel(const CgRun* __restrict__ runs, const int* __restrict__ start,
+                                                        int nruns, int* __restrict__ vr, int* __restrict__ vo) {
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (r >= nruns) return;
+  const int len = runs[r].l2 - runs[r].l1 + 1, s = start[r];
+  for (int j = threadIdx.x & 31; j < len; j += 32) {
+    vr[s + j] = r;
+    vo[s + j] = j;
   }
 }
 
@@ -682,16 +691,31 @@ __global__ void fixedge_axis_kernel(T* __restrict__ p, int n, int axis, int mode
   else if (axis == 1) { base = (size_t)a * n * n + b; stride = (size_t)n; }             // K=a, I=b
   else { base = (size_t)a * n + b; stride = (size_t)n * n; }                            // J=a, I=b
   auto L = [&](int t) -> T& { return p[base + (size_t)(t - 1) * stride]; };
-  const T z = (T)0;
-  if (mode == 1) {
-    for (int t = 1; t <= n - 1; ++t) if (L(t + 1) != z) { L(t) = L(t + 1); break; }
-    for (int t = n; t >= 2; --t) if (L(t - 1) != z) { L(t) = L(t - 1); break; }
-  } else if (mode == 2) {
-    for (int t = 2; t <= n - 1; ++t) if (L(t + 1) != z) { T v = L(t + 1); L(t) = v; L(t - 1) = v; break; }
-    for (int t = n - 1; t >= 2; --t) if (L(t - 1) != z) { T v = L(t - 1); L(t) = v; L(t + 1) = v; break; }
-  } else {
-    for (int t = 3; t <= n - 1; ++t) if (L(t + 1) != z) { T v = L(t + 1); L(t) = v; L(t - 1) = v; L(t - 2) = v; break; }
-    for (int t = n - 2; t >= 2; --t) if (L(t - 1) != z) { T v = L(t - 1); L(t) = v; L(t + 1) = v; L(t + 2) = v; break; }
+  // the first step i < m whose voxel at(i) is not zero (m if none), eight
+  // loads in flight at a time: the scan is bound by their latency
+  auto scan = [&](int m, auto at) {
+    for (int i = 0; i < m; i += 8) {
+      T v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = at(min(i + u, m - 1));
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (i + u < m && v[u] != (T)0) return i + u;
+    }
+    return m;
+  };
+  // forward: t = mode .. n-1 looks at t + 1; back: t = n (n - 1, n - 2) .. 2 at t - 1
+  const int fwd = n - mode, back = n - mode;
+  int i = scan(fwd, [&](int k) { return L(mode + 1 + k); });
+  if (i < fwd) {
+    const T v = L(mode + 1 + i);
+    for (int o = 0; o < mode; ++o) L(mode + i - o) = v;
+  }
+  const int top = n + 1 - mode;
+  i = scan(back, [&](int k) { return L(top - 1 - k); });
+  if (i < back) {
+    const T v = L(top - 1 - i);
+    for (int o = 0; o < mode; ++o) L(top - i + o) = v;
   }
 }
 
@@ -733,6 +757,13 @@ __global__ void widen_kernel(const float* __restrict__ in, T* __restrict__ out, 
     out[q] = (T)in[q];
 }
 
+// T -> float rounding copy
+template <class T>
+__global__ void narrow_kernel(const T* __restrict__ in, float* __restrict__ out, size_t count) {
+  for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < count; q += (size_t)gridDim.x * blockDim.x)
+    out[q] = (float)in[q];
+}
+
 void cg_release(spi_ctx* c) {
   for (auto& b : c->cg_buf) b.release();
   for (auto& b : c->cg_fbs) b.release();
@@ -753,21 +784,26 @@ static int cg_setup(spi_ctx* c, int n, float ri, CgProblem& pb) {
   pb.ldp = n / 2 + 1;
   pb.ri = ri;
   prepcub_s(n, ri, pb.ldp, pb.runs);
-  std::vector<int> vr, vo;
-  for (size_t r = 0; r < pb.runs.size(); ++r)
-    for (int j = pb.runs[r].l1; j <= pb.runs[r].l2; ++j) {
-      vr.push_back((int)r);
-      vo.push_back(j - pb.runs[r].l1);
-    }
-  pb.nvox = (long long)vr.size();
-  // cg_buf[0] runs, [1] vox_run, [2] vox_off
-  SPI_TRY(c->cg_buf[0].ensure(std::max<size_t>(1, pb.runs.size()) * sizeof(CgRun)));
-  SPI_TRY(c->cg_buf[1].ensure(std::max<size_t>(1, vr.size()) * sizeof(int)));
-  SPI_TRY(c->cg_buf[2].ensure(std::max<size_t>(1, vo.size()) * sizeof(int)));
-  if (!pb.runs.empty()) {
-    SPI_CUDA(cudaMemcpyAsync(c->cg_buf[0].p, pb.runs.data(), pb.runs.size() * sizeof(CgRun), cudaMemcpyHostToDevice, c->stream));
-    SPI_CUDA(cudaMemcpyAsync(c->cg_buf[1].p, vr.data(), vr.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-    SPI_CUDA(cudaMemcpyAsync(c->cg_buf[2].p, vo.data(), vo.size() * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+  // the runs, then the number of each one's first voxel
+  const size_t nr = pb.runs.size();
+  std::vector<CgRun> tab(pb.runs);
+  tab.resize(nr + (nr * sizeof(int) + sizeof(CgRun) - 1) / sizeof(CgRun));
+  int* start = reinterpret_cast<int*>(tab.data() + nr);
+  for (size_t r = 0; r < nr; ++r) {
+    start[r] = (int)pb.nvox;
+    pb.nvox += pb.runs[r].l2 - pb.runs[r].l1 + 1;
+  }
+  // cg_buf[0] runs and starts, [1] vox_run, [2] vox_off
+  SPI_TRY(c->cg_buf[0].ensure(std::max<size_t>(1, tab.size()) * sizeof(CgRun)));
+  SPI_TRY(c->cg_buf[1].ensure((size_t)std::max(1ll, pb.nvox) * sizeof(int)));
+  SPI_TRY(c->cg_buf[2].ensure((size_t)std::max(1ll, pb.nvox) * sizeof(int)));
+  if (nr > 0) {
+    SPI_CUDA(cudaMemcpyAsync(c->cg_buf[0].p, tab.data(), tab.size() * sizeof(CgRun), cudaMemcpyHostToDevice, c->stream));
+    const CgRun* d = c->cg_buf[0].as<CgRun>();
+    cg_voxels_kernel<<<(unsigned)((nr + 7) / 8), 256, 0, c->stream>>>(d, reinterpret_cast<const int*>(d + nr), (int)nr,
+                                                                      c->cg_buf[1].as<int>(), c->cg_buf[2].as<int>());
+    SPI_TRY(check_kernel("cg_voxels_kernel"));
+    c->count();
   }
   return 0;
 }
@@ -1681,15 +1717,15 @@ static int bpcg_run(spi_ctx* c, const float* projs, int n, int nang, const float
   if (exec) cudaGraphExecDestroy(exec);
   if (graph) cudaGraphDestroy(graph);
   if (niter_out) *niter_out = done;
-  // BCKN -> float volume (staged in the float projection buffer)
-  if (sizeof(T) == sizeof(float)) {
-    SPI_CUDA(cudaMemcpyAsync(vol_out, bckn, nnn * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
-  } else {
-    std::vector<T> tmp(nnn);
-    SPI_CUDA(cudaMemcpyAsync(tmp.data(), bckn, vb, cudaMemcpyDeviceToHost, c->stream));
-    SPI_CUDA(cudaStreamSynchronize(c->stream));
-    for (size_t i = 0; i < nnn; ++i) vol_out[i] = (float)tmp[i];
+  // BCKN -> float volume, rounded on the device into BCKE, which is free now
+  const float* res = reinterpret_cast<const float*>(bckn);
+  if (sizeof(T) != sizeof(float)) {
+    narrow_kernel<T><<<nnn_b, 256, 0, c->stream>>>(bckn, reinterpret_cast<float*>(bcke), nnn);
+    SPI_TRY(check_kernel("narrow_kernel"));
+    c->count();
+    res = reinterpret_cast<const float*>(bcke);
   }
+  SPI_CUDA(cudaMemcpyAsync(vol_out, res, nnn * sizeof(float), cudaMemcpyDeviceToHost, c->stream));
   SPI_CUDA(cudaStreamSynchronize(c->stream));
   return 0;
 }
