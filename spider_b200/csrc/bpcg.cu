@@ -350,7 +350,8 @@ __global__ void __launch_bounds__(256) cg_layout_kernel(const double* __restrict
 // mcap * 65535, and the pixel is hi * 65536 + lo exactly (a step of ~1e-11
 // max|x|).
 //
-// Bound: shared-memory wavefronts, eight atomics a voxel (WIDE).  A warp takes
+// Bound: instruction issue (84%), then shared-memory wavefronts (60%), eight
+// atomics a voxel (WIDE).  A warp takes
 // 32 neighbouring voxel lines along y or z (`groups`, longest first) and walks
 // them together in x, each lane with the reference's sequential XB/YB steps
 // from the start of its own run, so every sample lands where the reference
@@ -492,14 +493,15 @@ __device__ __forceinline__ double widen_nonneg(float f) {
 // image k at projt + (k - kbase) * n * n), accumulating in T, one thread a
 // voxel, the images in order.
 //
-// Bound: instruction issue and the converter unit.  `perm` lists the sphere's
-// voxels by 8 x 4 x 4 boxes, so that the table entries of a warp, and of the
+// Bound: instruction issue (80%) and the wavefronts of the gathers (75%).  `perm`
+// lists the sphere's voxels by 8 x 4 x 4 boxes of 2 x 2 x 2 cells, so that the table entries of a warp, and of the
 // warps of a block, lie together; the transforms come from shared memory, and
 // four entries are asked for before the first is used.  PREPCUB_S keeps RI +
 // MODE + 1 <= N/2 (a larger radius is refused before any result), so positions
 // lie in [2, N - 1] and truncation is rounding down, which adding 2^23 does.
-// At 128^3 3.4 -> 2.05 us an image against voxels in run order, transforms
-// from global memory and all conversions through the converter.
+// At 128^3 3.5 -> 2.5 us an image against voxels in run order, transforms from
+// global memory and all conversions through the converter (2.6 with the voxels
+// of a box in rows of 8).
 template <class T, bool WIDE>
 __global__ void __launch_bounds__(256) bckpj_projt_kernel(T* __restrict__ cube, const int2* __restrict__ lines,
                                                           const int* __restrict__ perm, int nvox,
@@ -880,9 +882,9 @@ static int projt_chunk(int n, int nang, size_t entry) {
 // into C row bands (1, 2, 4 or 8 CTAs per projection) when one CTA's 200 KB
 // do not hold it; 0 when no split does.  A split image takes twice the
 // fewest bands that fit: smaller bands put 3 CTAs on an SM instead of 1,
-// which outweighs walking every run once more per band (256^3, 2,000
-// images: mode 3 0.230 s per iteration with 4 bands against 0.254 s with 2
-// and 0.313 s with 8; mode 2 0.365 s with 8 against 0.411 s with 4).
+// which outweighs walking every line once more per band (256^3, 2,000
+// images: mode 3 0.134 s per iteration with 4 bands against 0.196 s with 2
+// and 0.162 s with 8; mode 2 0.175 s with 8 against 0.253 s with 4).
 // SPI_CG_BANDS forces a C at least the fewest that fit.
 static size_t band_bytes(int n, int C, bool wide) {
   if (C == 1) return (size_t)n * n * (wide ? 8 : 4);
@@ -927,26 +929,27 @@ static int launch_backproject_projt(spi_ctx* c, const CgProblem& pb, T* cube, co
   return 0;
 }
 
-// The sphere's voxels of 8 x 4 x 4 boxes, one warp a box and one lane a line
+// The sphere's voxels of 8 x 4 x 4 boxes, by 2 x 2 x 2 cells inside: the eight
+// lanes of a 16-byte load's pass project onto two or three pixel rows, wherever
+// the view comes from (eight voxels in x: up to eight).  One warp a box.
 __global__ void __launch_bounds__(256) cg_perm_kernel(const int2* __restrict__ lines, const int* __restrict__ start, int n,
                                                       int bx, int by, int nbox, int* __restrict__ perm) {
   const int box = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (box >= nbox) return;
-  const int x = box % bx * 8, y = box / bx % by * 4 + (lane & 3), z = box / bx / by * 4 + (lane >> 2);
-  int a = 0, e = 0;
-  if (lane < 16 && y < n && z < n) {
-    const int2 run = lines[z * n + y];
-    a = max(x, run.x);
-    e = min(x + 8, run.x + run.y);
+  int* out = perm + start[box];
+  for (int i = lane; i < 128; i += 32) {
+    const int x = box % bx * 8 + (i >> 2 & 6) + (i & 1);
+    const int y = box / bx % by * 4 + (i >> 4 & 2) + (i >> 1 & 1);
+    const int z = box / bx / by * 4 + (i >> 5 & 2) + (i >> 2 & 1);
+    bool in = false;
+    if (y < n && z < n) {
+      const int2 run = lines[z * n + y];
+      in = (unsigned)(x - run.x) < (unsigned)run.y;
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (in) out[__popc(m & ((1u << lane) - 1))] = (z * n + y) * n + x;
+    out += __popc(m);
   }
-  const int cnt = max(e - a, 0);
-  int before = cnt;
-  for (int o = 1; o < 16; o <<= 1) {
-    const int w = __shfl_up_sync(0xffffffffu, before, o);
-    if (lane >= o) before += w;
-  }
-  int* out = perm + start[box] + before - cnt;
-  for (int i = 0; i < cnt; ++i) out[i] = (z * n + y) * n + a + i;
 }
 
 // Tables of the projector of the mixed modes: cg_buf[8] = the run {first x,
