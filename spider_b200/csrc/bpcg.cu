@@ -20,6 +20,7 @@
 #include <atomic>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <unordered_map>
 
 #include "../../include/spider_b200.h"
@@ -493,15 +494,15 @@ __device__ __forceinline__ double widen_nonneg(float f) {
 // image k at projt + (k - kbase) * n * n), accumulating in T, one thread a
 // voxel, the images in order.
 //
-// Bound: instruction issue (80%) and the wavefronts of the gathers (75%).  `perm`
+// Bound: instruction issue and the wavefronts of the gathers, both near 80%.  `perm`
 // lists the sphere's voxels by 8 x 4 x 4 boxes of 2 x 2 x 2 cells, so that the table entries of a warp, and of the
 // warps of a block, lie together; the transforms come from shared memory, and
 // four entries are asked for before the first is used.  PREPCUB_S keeps RI +
 // MODE + 1 <= N/2 (a larger radius is refused before any result), so positions
 // lie in [2, N - 1] and truncation is rounding down, which adding 2^23 does.
-// At 128^3 3.5 -> 2.5 us an image against voxels in run order, transforms from
-// global memory and all conversions through the converter (2.6 with the voxels
-// of a box in rows of 8).
+// At 128^3 3.5 -> 2.1 us an image against voxels in run order, transforms from
+// global memory and all conversions through the converter (2.5 with each of the
+// four images guarded; 2.6 before with the voxels of a box in rows of 8).
 template <class T, bool WIDE>
 __global__ void __launch_bounds__(256) bckpj_projt_kernel(T* __restrict__ cube, const int2* __restrict__ lines,
                                                           const int* __restrict__ perm, int nvox,
@@ -523,36 +524,39 @@ __global__ void __launch_bounds__(256) bckpj_projt_kernel(T* __restrict__ cube, 
   T c = cube[lin];
   const float fx = (float)(run.x + 1 - ldp), fy = (float)(line % n + 1 - ldp), fz = (float)(line / n + 1 - ldp);
   const float fj = (float)(lin - line * n - run.x), fl = (float)ldp;
-  const int limit = n * n - n - 1;
-  const ProjtEntry<WIDE>* table = projt + (size_t)(k0 - kbase) * n * n - 1;
-  for (int k = 0; k < k1 - k0; k += 4) {
-    double b[4][4];
-    float dx[4], dy[4];
+  // PROJT column (iqy - 1) n + iqx, 0-based, from the bits of 2^23 + iq; any
+  // other goes to the last entry of a table, which is zero
+  const unsigned top = (unsigned)n * n - 1, c0 = 0u - 0x4b000001u * (unsigned)n - 0x4b000001u;
+  const ProjtEntry<WIDE>* table = projt + (size_t)(k0 - kbase) * n * n;
+  auto images = [&](int k, auto count) {   // images k .. k + count - 1 of the launch
+    constexpr int U = decltype(count)::value;
+    double b[U][4];
+    float dx[U], dy[U];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float4 mx = sx[min(k + u, 63)], my = sy[min(k + u, 63)];
+    for (int u = 0; u < U; ++u) {
+      const float4 mx = sx[k + u], my = sy[k + u];
       // XB = ((X-LDP)*DM1 + (Y-LDP)*DM2 + (Z-LDP)*DM3) + LDPNM ; XBB = XB + JT*DM1
       const float xb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, mx.x), __fmul_rn(fy, mx.y)), __fmul_rn(fz, mx.z)), fl);
       const float yb = __fadd_rn(__fadd_rn(__fadd_rn(__fmul_rn(fx, my.x), __fmul_rn(fy, my.y)), __fmul_rn(fz, my.z)), fl);
       const float xbb = __fadd_rn(xb, __fmul_rn(fj, mx.x));
       const float ybb = __fadd_rn(yb, __fmul_rn(fj, my.x));
       const float tx = __fadd_rd(xbb, 8388608.0f), ty = __fadd_rd(ybb, 8388608.0f);
-      const int iqx = __float_as_int(tx) & 0x7fffff, iqy = __float_as_int(ty) & 0x7fffff;
       dx[u] = __fsub_rn(xbb, __fsub_rn(tx, 8388608.0f));
       dy[u] = __fsub_rn(ybb, __fsub_rn(ty, 8388608.0f));
-      const int I = (iqy - 1) * n + iqx;  // PROJT column, 1-based
-      b[u][0] = b[u][1] = b[u][2] = b[u][3] = 0.0;
-      if (k + u < k1 - k0 && I >= 1 && I <= limit)
-        projt_load(table + (size_t)(k + u) * n * n + I, b[u][0], b[u][1], b[u][2], b[u][3]);
+      const unsigned I = __float_as_uint(ty) * (unsigned)n + __float_as_uint(tx) + c0;
+      projt_load(table + min(I, top), b[u][0], b[u][1], b[u][2], b[u][3]);
+      table += top + 1;
     }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (k + u < k1 - k0) {
-        const T ex = (T)widen_nonneg(dx[u]), ey = (T)widen_nonneg(dy[u]);
-        c = radd(radd(radd(c, (T)b[u][0]), rmul(ey, (T)b[u][1])), rmul(ex, radd((T)b[u][2], rmul(ey, (T)b[u][3]))));
-      }
+    for (int u = 0; u < U; ++u) {
+      const T ex = (T)widen_nonneg(dx[u]), ey = (T)widen_nonneg(dy[u]);
+      c = radd(radd(radd(c, (T)b[u][0]), rmul(ey, (T)b[u][1])), rmul(ex, radd((T)b[u][2], rmul(ey, (T)b[u][3]))));
     }
-  }
+  };
+  const int cnt = k1 - k0;
+  int k = 0;
+  for (; k + 4 <= cnt; k += 4) images(k, std::integral_constant<int, 4>());
+  for (; k < cnt; ++k) images(k, std::integral_constant<int, 1>());
   cube[lin] = c;
 }
 
