@@ -523,9 +523,9 @@ def fourier_cg_measure(ctx, projs, ang, K, lam=1e-3, check_images=1000, check_it
     xg = x[..., 0] + 1j * x[..., 1]
     out["rel_err_vs_fp64_oracle"] = float(np.linalg.norm(xg - xr) / np.linalg.norm(xr))
     out["check"] = f"{check_images} images, {check_iters} iterations, oracle FP64 CG {time.perf_counter() - t0:.1f} s"
-    out["operator"] = "FourierSlice (central-slice extraction) and ONELINE insertion without weights, fused " \
-                      "E^T E + lam I with FP64 sums and scatter (FP32 table weights), FP64 CG vectors; " \
-                      "fp32_operator: the same pass with FP32 sums"
+    out["operator"] = "FourierSlice (central-slice extraction) and ONELINE insertion without weights, " \
+                      "E^T E + lam I through a slice buffer with FP64 sums (FP32 table weights), FP64 CG vectors; " \
+                      "fp32_operator: the same with FP32 sums"
     return out
 
 

@@ -2,12 +2,12 @@
 //
 // Per chunk of images:   stage (PADD2 + phase as a circular shift, FP64 mean)
 //                        -> batched cuFFT R2C
-//                        -> insert (ONELINE, one persistent launch per chunk)
+//                        -> insert (ONELINE, one persistent launch per sub-batch)
 // Per volume:            SYMPLANE0 -> NRMW2 (+ADDADA) -> cuFFT C2R -> WINDKB2A
 //
 // The grid is an array of float4 {Re X, Im X, W, 0} voxels laid out
-// [k][j][i], i = 0..nx fastest (Fortran X(0:NX,N,N) with W interleaved), so
-// each gridding tap is one 16-byte vector atomic in L2.
+// [k][j][i], i = 0..nx fastest (Fortran X(0:NX,N,N) with W interleaved), so a
+// voxel's sum of one slice's taps is one 16-byte vector atomic in L2.
 #include <cuda_bf16.h>
 
 #include <algorithm>
