@@ -64,25 +64,14 @@ __global__ void __launch_bounds__(kExThreads) fs_extract_kernel(const T2* __rest
     T2* row = out + ((size_t)s * N + (J >= 0 ? J : N + J)) * rl;
     const float fj = (float)J;
     const float xj = __fmul_rn(fj, sd.dm[3]), yj = __fmul_rn(fj, sd.dm[4]), zj = __fmul_rn(fj, sd.dm[5]);
+    // a matrix that is not a rotation's (an angle that is not finite) has no taps: its rows are zero
+    const bool rotation = slab_rotation(sd.dm);
     int I0 = 0;
-    for (; I0 <= nx && I0 * I0 + J * J < nx * nx; I0 += 8) {   // warp-uniform
+    for (; rotation && I0 <= nx && I0 * I0 + J * J < nx * nx; I0 += 8) {   // warp-uniform
       const int I = I0 + g;
-      const float fi = (float)I;
-      float x = __fadd_rn(__fmul_rn(fi, sd.dm[0]), xj);
-      float y = __fadd_rn(__fmul_rn(fi, sd.dm[1]), yj);
-      float z = __fadd_rn(__fmul_rn(fi, sd.dm[2]), zj);
-      const bool flip = x < 0.0f;
-      if (flip) { x = -x; y = -y; z = -z; }
-      // inside the disc and ONELINE's bounds on the nearest voxel (pixels 6 inside the edge always are)
-      const int r2 = I * I + J * J;
-      bool ok = !(I == 0 && J < 0);
-      if (nx <= 6 || r2 > (nx - 6) * (nx - 6)) {
-        const float fn = (float)N;
-        const int ix = slab_floor(__fadd_rn(__fadd_rn(x, 0.5f), fn)) - N, iy = slab_floor(__fadd_rn(__fadd_rn(y, 0.5f), fn)) - N;
-        const int iz = slab_floor(__fadd_rn(__fadd_rn(z, 0.5f), fn)) - N;
-        ok = ok && r2 < nx * nx && ix <= nx - 3 && iy >= -nx + 4 && iy <= nx - 3 && iz >= -nx + 4 && iz <= nx - 3;
-      }
-      if (!ok) x = y = z = 0.0f;   // keeps the look-ups in range; no taps follow
+      float x, y, z;
+      bool flip;
+      const bool ok = slab_extract_pixel(sd.dm, xj, yj, zj, I, J, nx, x, y, z, flip);
       const int fx = slab_first(x), fy = slab_first(y), fz = slab_first(z);
       const float tx = tap(x, fx + q), tyq = tap(y, fy + q), tzq = tap(z, fz + q);
       // main tap (ixp, iyp, izp), or for ixp < 0 the reflected point with the conjugate value

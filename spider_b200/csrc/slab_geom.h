@@ -95,9 +95,18 @@ struct SlabFrame {
   float iau, iav;        // 1 / au, 1 / av (or a huge number)
 };
 
-// The frame of a slice with DM(1:6) = dm; false when the matrix is not a
-// rotation's (no finite normal), in which case the slice has no taps.
+// Are DM(1:3) and DM(4:6) = dm the unit vectors of a rotation?  An angle that is
+// not finite makes them NaN (CANG); such a slice has no taps, and its
+// coordinates must not become indices.
+SLAB_HD bool slab_rotation(const float* dm) {
+  const float a = dm[0] * dm[0] + dm[1] * dm[1] + dm[2] * dm[2], b = dm[3] * dm[3] + dm[4] * dm[4] + dm[5] * dm[5];
+  return a > 0.5f && a < 1.5f && b > 0.5f && b < 1.5f;   // false for NaN
+}
+
+// The frame of a slice with DM(1:6) = dm; false when they are not a rotation's,
+// in which case the slice has no taps.
 SLAB_HD bool slab_frame(const float* dm, SlabFrame& f) {
+  if (!slab_rotation(dm)) return false;
   const float n0 = dm[1] * dm[5] - dm[2] * dm[4], n1 = dm[2] * dm[3] - dm[0] * dm[5], n2 = dm[0] * dm[4] - dm[1] * dm[3];
   const float m0 = fabsf(n0), m1 = fabsf(n1), m2 = fabsf(n2);
   f.d = (m2 >= m0 && m2 >= m1) ? 2 : (m1 >= m0 ? 1 : 0);
@@ -205,6 +214,32 @@ SLAB_HD bool slab_inside(const SlabFrame& f, const SlabPix& p, int I, int J, int
   const int iw = slab_floor(sl_add(sl_add(sg * p.w, 0.5f), fn)) - 2 * nx;
   const int lo = -nx + 4, hi = nx - 3;
   return iu <= hi && iv <= hi && iw <= hi && iv >= lo && (f.d == 0 || iw >= lo) && (f.d != 0 || iu >= lo);
+}
+
+// Pixel (I, J), I >= 0, of a slice as the extraction takes it: at (x, y, z),
+// flipped where its x was negative; false, and at the origin, when it is outside
+// the disc or ONELINE's bounds on the nearest voxel.  (xj, yj, zj) = J DM(4:6).
+// Pixels 6 inside the edge are inside without a look, so the slice has to be a
+// rotation's (slab_rotation).
+SLAB_HD bool slab_extract_pixel(const float* dm, float xj, float yj, float zj, int I, int J, int nx, float& x, float& y,
+                                float& z, bool& flip) {
+  const float fi = (float)I;
+  x = sl_add(sl_mul(fi, dm[0]), xj);
+  y = sl_add(sl_mul(fi, dm[1]), yj);
+  z = sl_add(sl_mul(fi, dm[2]), zj);
+  flip = x < 0.0f;
+  if (flip) { x = -x; y = -y; z = -z; }
+  const int r2 = I * I + J * J;
+  bool ok = !(I == 0 && J < 0);
+  if (nx <= 6 || r2 > (nx - 6) * (nx - 6)) {
+    const int N = 2 * nx;
+    const float fn = (float)N;
+    const int ix = slab_floor(sl_add(sl_add(x, 0.5f), fn)) - N, iy = slab_floor(sl_add(sl_add(y, 0.5f), fn)) - N;
+    const int iz = slab_floor(sl_add(sl_add(z, 0.5f), fn)) - N;
+    ok = ok && r2 < nx * nx && ix <= nx - 3 && iy >= -nx + 4 && iy <= nx - 3 && iz >= -nx + 4 && iz <= nx - 3;
+  }
+  if (!ok) x = y = z = 0.0f;   // keeps look-ups in range
+  return ok;
 }
 
 // first of the four voxels along an axis that hold every nonzero tap of

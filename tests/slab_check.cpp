@@ -5,7 +5,12 @@
 //
 //   slab_check NX SEED COUNT   ->  one line per rotation:
 //   kind banks max_rows max_pixels taps_direct taps_columns bad
-// `bad` counts voxels whose set of (pixel, weight bits) differs, taps outside
+//   slab_check extract NX SEED COUNT   ->  bad
+// counts look-ups and voxels of the extraction's pixels that are out of range, and
+// matrices with an element or angle that is not finite which are taken for a
+// rotation's.
+//
+// `bad` of the first form counts voxels whose set of (pixel, weight bits) differs, taps outside
 // their column's voxel range, tiles over the capacity, and pixel rows or spans
 // that do not cover a tap.
 #include <cstdint>
@@ -76,7 +81,69 @@ static long long direct(const float* dm, int nx, Taps& t) {
   return n;
 }
 
+// CANG in REAL (cang.f:44-81)
+static void euler(float ps, float th, float ph, float* dm) {
+  const float r = 3.14159265358979323846f / 180.0f;
+  const float cp = std::cos(ps * r), sp = std::sin(ps * r), ct = std::cos(th * r), st = std::sin(th * r);
+  const float cf = std::cos(ph * r), sf = std::sin(ph * r);
+  const float m[6] = {cf * ct * cp - sf * sp, sf * ct * cp + cf * sp, -st * cp,
+                      -cf * ct * sp - sf * cp, -sf * ct * sp + cf * cp, st * sp};
+  memcpy(dm, m, sizeof(m));
+}
+
+// The extraction's windows (fs_extract.cuh): four lanes per pixel, 4 x 4 (y, z) voxels each
+static int extract(int nx, unsigned seed, int count) {
+  const int N = 2 * nx, kExTab = 3336;
+  const long long rl = nx + 1, total = rl * N * N;
+  const float fltb = 4999.0f / 3.0f, last = 1.8f * fltb;
+  std::mt19937 rng(seed);
+  std::uniform_real_distribution<float> U(0.0f, 1.0f);
+  long long bad = 0;
+  for (int q = 0; q < count; ++q) {
+    const float d[3] = {q < 4 ? 90.0f * q : 360.0f * U(rng), q < 16 ? 45.0f * (q / 4) : 180.0f * U(rng), q < 8 ? 45.0f : 360.0f * U(rng)};
+    float dm[6];
+    euler(d[0], d[1], d[2], dm);
+    SlabFrame f;
+    if (!slab_rotation(dm) || !slab_frame(dm, f)) ++bad;
+    for (float v : {NAN, INFINITY, -INFINITY})
+      for (int e = 0; e < 9; ++e) {   // an angle, or an element of the matrix
+        float b[6], a[3] = {d[0], d[1], d[2]};
+        if (e < 3) { a[e] = v; euler(a[0], a[1], a[2], b); }
+        else { memcpy(b, dm, sizeof(b)); b[e - 3] = v; }
+        if (slab_rotation(b) || slab_frame(b, f)) ++bad;
+      }
+    for (int J = -nx + 1; J <= nx; ++J)
+      for (int I0 = 0; slab_rotation(dm) && I0 <= nx && I0 * I0 + J * J < nx * nx; I0 += 8)
+        for (int I = I0; I < I0 + 8; ++I) {
+          float c[3];
+          bool flip;
+          const float fj = (float)J;
+          const bool ok = slab_extract_pixel(dm, fj * dm[3], fj * dm[4], fj * dm[5], I, J, nx, c[0], c[1], c[2], flip);
+          float t[3][4];
+          int first[3];
+          for (int a = 0; a < 3; ++a) {
+            first[a] = slab_first(c[a]);
+            for (int l = 0; l < 4; ++l) {
+              const int i = slab_nint(fabsf(c[a] - (float)(first[a] + l)) * fltb);
+              if (i < 0 || i >= kExTab) ++bad;
+              t[a][l] = (float)i <= last ? 1.0f : 0.0f;
+            }
+          }
+          for (int e = 0; ok && e < 64; ++e) {
+            const int l = e & 3, m = (e >> 2) & 3, k = e >> 4, x = first[0] + l;
+            if (t[0][l] * t[1][m] * t[2][k] == 0.0f) continue;
+            const int y = x < 0 ? -(first[1] + m) : first[1] + m, z = x < 0 ? -(first[2] + k) : first[2] + k;
+            const long long i = ((z < 0 ? N + z : z) * (long long)N + (y < 0 ? N + y : y)) * rl + (x < 0 ? -x : x);
+            if (i < 0 || i >= total || y < -N || y >= N || (x < 0 ? -x : x) >= nx) ++bad;
+          }
+        }
+  }
+  printf("%lld\n", bad);
+  return 0;
+}
+
 int main(int argc, char** argv) {
+  if (argc == 5) return extract(atoi(argv[2]), atoi(argv[3]), atoi(argv[4]));
   const int nx = atoi(argv[1]), count = atoi(argv[3]);
   std::mt19937 rng(atoi(argv[2]));
   // a stand-in for FILLBESSIL's table with its support: nonzero up to 1.8, zero beyond

@@ -28,3 +28,11 @@ def test_columns_find_every_tap(check, nx, count):
         assert nrows <= 47 and npix <= 654
     assert {r[0] for r in rows} == {0, 1, 2}        # every dominant axis
     assert {r[1] for r in rows} == {2, 3}           # shallow and steep slices
+
+
+@pytest.mark.parametrize("nx,count", [(8, 60), (9, 60), (33, 30), (150, 17), (512, 3)])
+def test_extraction_stays_in_range(check, nx, count):
+    """Every table entry and voxel of the extraction's windows is in range, and a
+    matrix with a NaN or infinite angle or element is not taken for a rotation."""
+    out = subprocess.run([check, "extract", str(nx), "7", str(count)], check=True, capture_output=True, text=True).stdout
+    assert int(out) == 0

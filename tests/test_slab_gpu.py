@@ -119,3 +119,34 @@ def test_fourier_slice_normal_workspaces(ctx):
                                               st) == 101
     finally:
         plan.close()
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_fourier_slice_angles_not_finite(ctx, bad):
+    """A slice with an angle that is not finite has no taps: E writes zeros, E^T and
+    the normal operators leave it out, the other slices are as without it."""
+    import torch
+
+    from spider_b200 import autograd
+    nx = 24
+    good = _angles(12, 6)
+    ang = np.repeat(good, 2, axis=0)
+    for i in range(12):
+        ang[2 * i + 1, i % 3] = bad
+    X = torch.randn((2 * nx, 2 * nx, nx + 1, 2), device="cuda")
+    T = torch.randn((24, 2 * nx, nx + 1, 2), device="cuda")
+    plan, ref = autograd.FourierSlicePlan(nx, ang, ctx=ctx), autograd.FourierSlicePlan(nx, good, ctx=ctx)
+    try:
+        for fwd, x in (("forward", X), ("forward64", X.double())):
+            got = getattr(plan, fwd)(x)
+            assert torch.equal(got[::2], getattr(ref, fwd)(x))
+            assert not got[1::2].any()
+        for op, args, rargs, tol in (("adjoint", (T,), (T[::2].contiguous(),), 2e-6),
+                                     ("adjoint64", (T,), (T[::2].contiguous(),), 1e-12),
+                                     ("normal", (X, 0.25), (X, 0.25), 2e-6),
+                                     ("normal64", (X.double(), 0.25), (X.double(), 0.25), 1e-12)):
+            got, want = getattr(plan, op)(*args), getattr(ref, op)(*rargs)
+            assert ((got - want).norm() / want.norm()).item() <= tol, op
+    finally:
+        plan.close()
+        ref.close()
