@@ -510,18 +510,21 @@ __global__ void __launch_bounds__(256) bckpj_projt_kernel(T* __restrict__ cube, 
                                                           const CgDM* __restrict__ dms, int kbase, int k0, int k1, int n,
                                                           int ldp) {
   __shared__ float4 sx[64], sy[64];   // {DM1, DM2, DM3, -}, {DM4, DM5, DM6, -}
+  bool lost = false;   // a transform is not finite (its angles are not)
   if (threadIdx.x < k1 - k0) {
     const CgDM dm = dms[k0 + threadIdx.x];
     sx[threadIdx.x] = make_float4(dm.d[0], dm.d[1], dm.d[2], 0.0f);
     sy[threadIdx.x] = make_float4(dm.d[3], dm.d[4], dm.d[5], 0.0f);
+    lost = !isfinite(dm.d[0] + dm.d[1] + dm.d[2] + dm.d[3] + dm.d[4] + dm.d[5]);
   }
-  __syncthreads();
+  lost = __syncthreads_or(lost);
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvox) return;
   const int lin = perm[v];
   const int line = lin / n;
   const int2 run = lines[line];
-  T c = cube[lin];
+  // a position that is not finite makes the sum NaN; the integer forms below would lose that
+  T c = lost ? (T)NAN : cube[lin];
   const float fx = (float)(run.x + 1 - ldp), fy = (float)(line % n + 1 - ldp), fz = (float)(line / n + 1 - ldp);
   const float fj = (float)(lin - line * n - run.x), fl = (float)ldp;
   // PROJT column (iqy - 1) n + iqx, 0-based, from the bits of 2^23 + iq; any

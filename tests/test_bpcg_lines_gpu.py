@@ -39,3 +39,20 @@ def test_mixed_operators_match_fp64(ctx, monkeypatch, n, ri, bands, prec, tol):
     assert len(log) == len(rlog)
     assert np.abs(ref).max() > 0
     assert np.abs(v - ref).max() <= tol * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("prec", ["mixed64", "mixed", "fast"])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_mixed_angle_not_finite(ctx, bad, prec):
+    """A direction with an angle that is not finite is not passed over: the volume is
+    NaN where the FP64 operators' is."""
+    g = np.random.default_rng(5)
+    n, m = 24, 70
+    img = g.standard_normal((m, n, n)).astype(np.float32)
+    ang = np.stack([g.uniform(0, 360, m), np.degrees(np.arccos(g.uniform(-1, 1, m))), g.uniform(0, 360, m)], 1).astype(np.float32)
+    ang[66, 0] = bad   # psi; HIANG takes phi and theta alone, so the merged directions stay finite
+    kw = dict(errm=1e-30, chim=0.0, maxit=2, mode=1, lam=0.5, ctx=ctx)
+    v, _ = ops.bpcg(img, ang, 9.0, fp64=prec, **kw)
+    ref, _ = ops.bpcg(img, ang, 9.0, fp64=True, **kw)
+    assert np.isnan(ref).any()
+    assert np.array_equal(np.isnan(v), np.isnan(ref))
