@@ -1657,6 +1657,7 @@ void bp_release(spi_ctx* c) {
   if (c->plan3d) cufftDestroy(c->plan3d);
   c->plan3d = 0;
   c->plan3d_n = 0;
+  c->fft_work.release();
   c->nx = c->n = c->ngrids = 0;
   c->pending_sym0[0] = c->pending_sym0[1] = false;
   c->merged = false;
@@ -1788,7 +1789,7 @@ void spi_ctx::phase_collect() {
 long long spi_ctx::device_bytes() const {
   long long t = 0;
   const DevBuf* bufs[] = {&grid[0], &grid[1], &part[0], &part[1], &comp[0], &comp[1], &kbtab, &imgs, &padded, &spectra, &spec_tmp, &slices, &cplx, &real3,
-                          &workctr,
+                          &workctr, &fft_work,
                           &wkb, &acc, &volbuf, &pj_vol, &pj_out, &pj_runs, &pj_dm, &pj_rows, &pj_v4, &pj_fbs};
   for (auto b : bufs) t += (long long)b->bytes;
   for (auto& b : cg_buf) t += (long long)b.bytes;
@@ -2148,10 +2149,35 @@ static int fft_batch(const spi_ctx* c, int m) {
   return std::min(b, c->sub);
 }
 
-// The R2C plan of `batch` images of the open reconstruction's size; the
-// least recently used of kPlans2d makes room for a new one.
+// The plans of a context take one work area in turn (each runs after the other
+// on the context's streams), sized by the largest.  A plan without a work area
+// of its own is host data, so all batch sizes of fft_batch (19 up to 8,192 images)
+// keep theirs: making one takes about as long as the transform of a small call.
+static int make_plan(spi_ctx* c, int rank, int n, cufftType type, int batch, cufftHandle* out) {
+  int dims[3] = {n, n, n};
+  size_t bytes = 0;
+  cufftHandle h = 0;
+  SPI_CUFFT(cufftCreate(&h));
+  cufftResult r = cufftSetAutoAllocation(h, 0);
+  if (r == CUFFT_SUCCESS)
+    r = rank == 2 ? cufftMakePlanMany(h, 2, dims, nullptr, 1, n * n, nullptr, 1, n * (n / 2 + 1), type, batch, &bytes)
+                  : cufftMakePlan3d(h, n, n, n, type, &bytes);
+  int st = 0;
+  if (r != CUFFT_SUCCESS) st = fail(kCufft, "cuFFT plan (n = %d, batch %d): error %d", n, batch, (int)r);
+  if (!st) st = c->fft_work.ensure(std::max<size_t>(bytes, 256));
+  if (st) {
+    cufftDestroy(h);
+    return st;
+  }
+  *out = h;
+  return 0;
+}
+
+// The R2C plan of `batch` images of the open reconstruction's size; the least
+// recently used of kPlans2d (more than fft_batch's sizes: SPI_BP_SUB may add others
+// to a context that stays open) makes room for a new one.
 static int plan2d_of(spi_ctx* c, int batch, cufftHandle* out) {
-  constexpr size_t kPlans2d = 4;
+  constexpr size_t kPlans2d = 32;
   auto& v = c->plans2d;
   for (size_t i = 0; i < v.size(); ++i)
     if (v[i].n == c->n && v[i].batch == batch) {
@@ -2159,15 +2185,13 @@ static int plan2d_of(spi_ctx* c, int batch, cufftHandle* out) {
       *out = v[0].plan;
       return 0;
     }
-  const int n = c->n;
-  int dims[2] = {n, n};
   cufftHandle h = 0;
-  SPI_CUFFT(cufftPlanMany(&h, 2, dims, nullptr, 1, n * n, nullptr, 1, n * (n / 2 + 1), CUFFT_R2C, batch));
+  SPI_TRY(make_plan(c, 2, c->n, CUFFT_R2C, batch, &h));
   if (v.size() == kPlans2d) {
     cufftDestroy(v.back().plan);
     v.pop_back();
   }
-  v.insert(v.begin(), spi_ctx::Plan2d{h, n, batch});
+  v.insert(v.begin(), spi_ctx::Plan2d{h, c->n, batch});
   *out = h;
   return 0;
 }
@@ -2175,6 +2199,7 @@ static int exec_r2c(spi_ctx* c, cudaStream_t st, int batch, float* in, float2* o
   cufftHandle h = 0;
   SPI_TRY(plan2d_of(c, batch, &h));
   SPI_CUFFT(cufftSetStream(h, st));
+  SPI_CUFFT(cufftSetWorkArea(h, c->fft_work.p));
   SPI_CUFFT(cufftExecR2C(h, in, reinterpret_cast<cufftComplex*>(out)));
   return 0;
 }
@@ -2939,7 +2964,7 @@ static int finish_one(spi_ctx* c, int ga, int gb, float* dvol) {
   if (c->plan3d == 0 || c->plan3d_n != n) {
     if (c->plan3d) cufftDestroy(c->plan3d);
     c->plan3d = 0;
-    SPI_CUFFT(cufftPlan3d(&c->plan3d, n, n, n, CUFFT_C2R));
+    SPI_TRY(make_plan(c, 3, n, CUFFT_C2R, 1, &c->plan3d));
     SPI_CUFFT(cufftSetStream(c->plan3d, c->stream));
     c->plan3d_n = n;
   }
@@ -2950,6 +2975,7 @@ static int finish_one(spi_ctx* c, int ga, int gb, float* dvol) {
   c->phase_end(ev);
   c->count();
   ev = c->phase_begin(5);
+  SPI_CUFFT(cufftSetWorkArea(c->plan3d, c->fft_work.p));
   SPI_CUFFT(cufftExecC2R(c->plan3d, reinterpret_cast<cufftComplex*>(c->cplx.p), c->real3.as<cufftReal>()));
   c->phase_end(ev);
   // WINDKB2A: |WKB| table and shell voxel count depend on nx only

@@ -74,6 +74,7 @@ struct spi_ctx {
   spi::HostBuf hslices;
   struct Plan2d { cufftHandle plan; int n, batch; };
   std::vector<Plan2d> plans2d;        // batched R2C plans, most recently used first
+  spi::DevBuf fft_work;               // work area of all plans2d and plan3d (they run in turn)
   int fft_own = 0;                    // 1 = the library's own two-pass R2C (power-of-two n), 0 = cuFFT
   spi::DevBuf fft_tw;                 // float2 W_n^t, t < n/2 (FP64-computed twiddles of the own R2C)
   cufftHandle plan3d = 0;

@@ -58,3 +58,35 @@ def test_reconstruction_after_another(end, fold_every):
                 assert synth.rel_l2(got[k], v) <= 2e-6, (first, second, k)
     finally:
         c.close()
+
+
+@pytest.mark.parametrize("nx", [24, 147])
+def test_calls_of_many_sizes(nx):
+    """Calls of seven sizes in turn, each with its own transform batch: the result is that
+    of one call of all images, and the plans share one work area, so that after the
+    largest call the others take no more device memory."""
+    import torch
+    sizes = (7, 20, 30, 45, 60, 90, 120)
+    m = sum(sizes)
+    rng = np.random.default_rng(nx)
+    imgs = rng.standard_normal((m, nx, nx)).astype(np.float32)
+    ang = synth.so3_angles(m, rng)
+    c, one = ops.Context(0), ops.Context(0)
+    try:
+        one.bp_open(nx, 1)
+        one.bp_insert(imgs, ang)
+        ref = one.bp_finish(("all",))["all"]
+        for turn in range(2):
+            c.bp_open(nx, 1)
+            end, free = m, []
+            for s in sorted(sizes, reverse=True):
+                c.bp_insert(imgs[end - s:end], ang[end - s:end])
+                end -= s
+                free.append(torch.cuda.mem_get_info()[0])
+            assert turn == 0 or len(set(free)) == 1
+            if turn == 0:
+                assert free[0] - free[-1] < 2 << 20   # the plans' constants, no work areas
+            assert synth.rel_l2(c.bp_finish(("all",))["all"], ref) <= 2e-6
+    finally:
+        c.close()
+        one.close()
