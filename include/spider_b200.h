@@ -191,9 +191,10 @@ int spi_bp_partial_out(spi_ctx* ctx, int g, float* x_out, float* w_out);
 int spi_bp_partial_add(spi_ctx* ctx, int g, const float* x_in, const float* w_in);
 
 /* End the open reconstruction and release its grids and chunk buffers.  When
- * they take at most 512 MB in all they stay with the context, so that a next
- * reconstruction of the same box size need not allocate and plan again; opening
- * another size, or destroying the context, releases them. */
+ * they take at most 512 MB in all (device memory with the transforms' work
+ * area, and pinned descriptors) they stay with the context, so that a next
+ * reconstruction of the same box size need not allocate and plan again;
+ * opening another size, or destroying the context, releases them. */
 int spi_bp_close(spi_ctx* ctx);
 
 /* One-shot BP 3F on host arrays (BP3F(.FALSE.,.FALSE.), bp3f.f:79). */

@@ -90,3 +90,27 @@ def test_calls_of_many_sizes(nx):
     finally:
         c.close()
         one.close()
+
+
+@pytest.mark.parametrize("nx,images,kept", [(64, 200, True), (83, 1100, False), (128, 200, False)])
+def test_close_keeps_at_most_its_limit(nx, images, kept):
+    """A closed reconstruction leaves at most 512 MB with its context: at 64^3 it stays
+    whole; 1,100 images at 83^3 stay below with their buffers but not with the
+    transforms' work area (166 = 2 x 83 takes one), 200 at 128^3 with neither."""
+    rng = np.random.default_rng(nx)
+    imgs = rng.standard_normal((images, nx, nx)).astype(np.float32)
+    c = ops.Context(0)
+    try:
+        empty = c.device_bytes
+        c.bp_open(nx, 1)
+        c.bp_insert(imgs, synth.so3_angles(images, rng))
+        c.bp_finish(("all",))
+        full = c.device_bytes
+        c.bp_close()
+        held = c.device_bytes
+        if kept:
+            assert held == full <= 512 << 20
+        else:
+            assert full > 512 << 20 and held - empty < 1 << 20
+    finally:
+        c.close()
