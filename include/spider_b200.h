@@ -149,7 +149,8 @@ int spi_bp_flush(spi_ctx* ctx);
 int spi_bp_autotune(spi_ctx* ctx, int force);
 
 /* The insertion launch in use: kernel (0 tile, 1 direct, 2 five x-tap lanes,
- * 3 four lanes over the nonzero window), threads per CTA, CTAs per SM, and
+ * 3 voxel columns, 4 tile in fixed point), threads per CTA (kernel 3: those
+ * that sum, always 128; a producer warp works beside them), CTAs per SM, and
  * the autotuner's time of one sample launch in ms (0 when not tuned). */
 int spi_bp_get_launch(const spi_ctx* ctx, int* kernel, int* threads, int* blocks_per_sm, float* tuned_ms);
 

@@ -1988,7 +1988,9 @@ int spi_bp_open(spi_ctx* c, int nx, int ngrids, const float* sym_angles, int nsy
       def_bps = kSlabBlocks;
     }
     c->insert_threads = env_int("SPI_INSERT_THREADS", def_threads);
-    if (c->insert_threads != 64 && c->insert_threads != 128 && c->insert_threads != 256 && c->insert_threads != 512)
+    // the column kernel's CTA is fixed (a tile's columns, two per thread, and the producer warp)
+    if (c->insert_mode == 3 || (c->insert_threads != 64 && c->insert_threads != 128 && c->insert_threads != 256 &&
+                                c->insert_threads != 512))
       c->insert_threads = def_threads;
     c->insert_blocks_per_sm = env_int("SPI_INSERT_BLOCKS_PER_SM", def_bps);
   }

@@ -334,6 +334,23 @@ def test_bp_autotune(ctx, orc):
         ctx.bp_close()
 
 
+@pytest.mark.parametrize("kernel,threads", [(None, 128), ("xlane", 512)])
+def test_reported_launch_is_the_one_used(ctx, monkeypatch, kernel, threads):
+    """spi_bp_get_launch reports a kernel's own CTA size: SPI_INSERT_THREADS sets that of
+    the per-tap kernels, the column kernel's is fixed."""
+    import ctypes
+    monkeypatch.setenv("SPI_INSERT_THREADS", "512")
+    if kernel:
+        monkeypatch.setenv("SPI_INSERT", kernel)
+    ctx.bp_open(24, 1)
+    try:
+        got = ctypes.c_int()
+        ops.check(ctx._L.spi_bp_get_launch(ctx.handle, None, ctypes.byref(got), None, None))
+        assert got.value == threads
+    finally:
+        ctx.bp_close()
+
+
 def test_bp3f_max_box_linearity(ctx):
     """At the largest box (nx = 512: a 1024^3 padded grid of 8.6 GB) the
     reconstruction is linear in the images for fixed angles (X is, W depends
