@@ -109,8 +109,9 @@ class FourierSlicePlan:
     [2nx, 2nx, nx+1, 2] (complex as (re, im) pairs), slices [nang, 2nx, nx+1, 2]
     in the layout and sign of the staged image spectra (``stage``).  forward,
     adjoint and normal run on torch's current stream, allocate nothing in the
-    library (normal's buffer comes from torch's allocator) and do not
-    synchronise, so they can be captured in a CUDA graph."""
+    library (normal's buffer comes from torch's allocator, under capture from
+    the pool of torch.cuda.graph) and do not synchronise, so they can be
+    captured in a CUDA graph."""
 
     def __init__(self, nx: int, angles, ctx: ops.Context | None = None, device: int = 0):
         import ctypes
@@ -167,12 +168,19 @@ class FourierSlicePlan:
 
     def _normal(self, grid, lam, out):
         """E^T (E grid) + lam grid through a slice buffer from torch's allocator: one per
-        call, on the call's stream, so calls on several streams do not share it."""
+        call, on the call's stream, so calls on several streams do not share it.  Where
+        there is no room for one, the form that keeps no slices runs instead."""
         import ctypes
         fp64 = int(grid.dtype == torch.float64)
         nb = ctypes.c_longlong()
         ops.check(self._L.spi_fslice_normal_ws_bytes(self._h, fp64, ctypes.byref(nb)))
-        ws = torch.empty(nb.value, dtype=torch.uint8, device=self.device)
+        try:
+            ws = torch.empty(nb.value, dtype=torch.uint8, device=self.device)
+        except torch.OutOfMemoryError:
+            one_pass = self._L.spi_fslice_normal64 if fp64 else self._L.spi_fslice_normal
+            ops.check(one_pass(self._h, ctypes.c_void_p(grid.data_ptr()), float(lam), ctypes.c_void_p(out.data_ptr()),
+                               self._stream()))
+            return out
         ops.check(self._L.spi_fslice_normal_ws(self._h, ctypes.c_void_p(grid.data_ptr()), float(lam),
                                                ctypes.c_void_p(out.data_ptr()), fp64, ctypes.c_void_p(ws.data_ptr()),
                                                nb.value, self._stream()))

@@ -121,6 +121,31 @@ def test_fourier_slice_normal_workspaces(ctx):
         plan.close()
 
 
+def test_fourier_slice_normal_without_room(ctx):
+    """Where torch cannot give the slice buffer (58 MB), the normal operator runs
+    without one, as it did before it had one."""
+    import torch
+
+    from spider_b200 import autograd
+    nx, nang = 24, 3000
+    plan = autograd.FourierSlicePlan(nx, _angles(nang, 8), ctx=ctx)
+    try:
+        x = torch.randn(plan.shape, dtype=torch.float64, device="cuda")
+        ref, got = torch.empty_like(x), torch.empty_like(x)
+        plan.normal64(x, 0.5, out=ref)
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        total = torch.cuda.get_device_properties(0).total_memory
+        torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (1 << 20)) / total)
+        try:
+            plan.normal64(x, 0.5, out=got)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0)
+        assert ((got - ref).norm() / ref.norm()).item() <= 1e-12
+    finally:
+        plan.close()
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
 def test_fourier_slice_angles_not_finite(ctx, bad):
     """A slice with an angle that is not finite has no taps: E writes zeros, E^T and
