@@ -361,8 +361,10 @@ __global__ void __launch_bounds__(256) cg_layout_kernel(const double* __restrict
 // `stride` words apart (1 or 31 mod 32) and are stored mirrored where the lines
 // run against that skew, so that neighbouring lanes fall into neighbouring
 // banks at any angle.  The volume is read from the layout in which the lanes'
-// voxels are contiguous (cg_layout_kernel).  At 128^3 with 1,000 directions 12.8 -> 3.9 us a projection against
-// one run a thread in run order (rows of n words, uncoalesced FP64 voxels).
+// voxels are contiguous (cg_layout_kernel), or, where there was no room for the
+// layouts, from the volume itself with a row or a plane between lanes.  At 128^3
+// with 1,000 directions 12.8 -> 3.9 us a projection against one run a thread in
+// run order (rows of n words, uncoalesced FP64 voxels).
 //
 // BAND (images too large for one CTA's shared memory): C CTAs per projection,
 // CTA b owning the pixel rows [b R, b R + R) (R = ceil(n / C)) and accumulating
@@ -372,9 +374,9 @@ __global__ void __launch_bounds__(256) cg_layout_kernel(const double* __restrict
 // others end once past it; integer sums make the tables identical to those of
 // one CTA.  (A 2-4 CTA cluster adding into one another's bands through
 // distributed shared memory was measured 3-8x slower at n = 256.)
-template <bool WIDE, bool WT, bool BAND>
+template <bool WIDE, bool WT, bool BAND, bool LAYOUTS>
 __global__ void __launch_bounds__(BAND ? 512 : 1024) prjcq_projt_kernel(
-    const double* __restrict__ layouts, const int2* __restrict__ lines, const int2* __restrict__ groups, int ngroups,
+    const double* __restrict__ volume, const int2* __restrict__ lines, const int2* __restrict__ groups, int ngroups,
     const CgDM* __restrict__ dms, const int* __restrict__ lb, int kbase, int n, int stride, int ldp, int C,
     const unsigned long long* __restrict__ maxabs_bits, float mcap, ProjtEntry<WT>* __restrict__ projt) {
   const int R = BAND ? (n + C - 1) / C : n;
@@ -409,7 +411,9 @@ __global__ void __launch_bounds__(BAND ? 512 : 1024) prjcq_projt_kernel(
   const int step = mirror ? -1 : 1;
   int* const origin = hi + (mirror ? n - 1 : 0);
   const size_t nn = (size_t)n * n;
-  const double* const vol = layouts + (along_y ? 0 : nn * n);
+  // voxel (x, t, f) of the lanes' coordinate t and the group's f lies at vol + f * sf + t * st + x * sx
+  const double* const vol = volume + (LAYOUTS && !along_y ? nn * n : 0);
+  const size_t sx = LAYOUTS ? nn : 1, sf = LAYOUTS || !along_y ? (size_t)n : nn, st = LAYOUTS ? 1 : along_y ? (size_t)n : nn;
   const int lane = threadIdx.x & 31;
   for (int g = threadIdx.x >> 5; g < ngroups; g += blockDim.x >> 5) {
     const int2 G = groups[g];
@@ -433,13 +437,13 @@ __global__ void __launch_bounds__(BAND ? 512 : 1024) prjcq_projt_kernel(
     }
     const int first = __reduce_min_sync(0xffffffffu, run.y > 0 ? run.x : n);
     const int last = __reduce_max_sync(0xffffffffu, run.y > 0 ? run.x + run.y : 0);
-    const double* src = vol + (size_t)G.x * n + t;
+    const double* src = vol + (size_t)G.x * sf + t * st;
     auto voxel = [&](int x, double loaded) {
       if ((unsigned)(x - run.x) >= (unsigned)run.y) return;
       const int iqx = __float2int_rz(xb), iqy = __float2int_rz(yb);
       const bool here = !BAND || (iqy >= r0 && iqy - 1 < h1);
       if (here && iqx >= 1 && iqx < n && iqy >= 1 && iqy < n) {
-        double cv = BAND ? __ldg(src + x * nn) : loaded;
+        double cv = BAND ? __ldg(src + x * sx) : loaded;
         // infinities (scale 0) and NaN add nothing, in WIDE as by conversion
         if (WIDE && !(fabs(cv) <= 1.7976931348623157e308)) cv = 0.0;
         const double dx = (double)__fsub_rn(xb, (float)iqx);
@@ -465,7 +469,7 @@ __global__ void __launch_bounds__(BAND ? 512 : 1024) prjcq_projt_kernel(
       for (int x = first; x < last; x += 4) {
         double c[4];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) c[u] = __ldg(src + min(x + u, n - 1) * nn);
+        for (int u = 0; u < 4; ++u) c[u] = __ldg(src + min(x + u, n - 1) * sx);
 #pragma unroll
         for (int u = 0; u < 4; ++u) voxel(x + u, c[u]);
       }
@@ -962,7 +966,7 @@ __global__ void __launch_bounds__(256) cg_perm_kernel(const int2* __restrict__ l
 // Tables of the projector of the mixed modes: cg_buf[8] = the run {first x,
 // voxels} of each line [n][n], then the groups {f, t} of 32 lines t .. t+31 at
 // the other coordinate f, longest first, then the sphere's voxels by 8 x 4 x 4
-// boxes (0-based linear indices); cg_buf[9] = room for the two layouts.
+// boxes (0-based linear indices).
 // The table is the same for (y, z) and (z, y): PREPCUB_S compares sums of
 // squared integers, which are exact.
 static int cg_lines(spi_ctx* c, CgProblem& pb) {
@@ -995,7 +999,6 @@ static int cg_lines(spi_ctx* c, CgProblem& pb) {
   for (int i = 0; i < (nbox + 1) / 2; ++i) tab.push_back(make_int2(start[2 * i], start[2 * i + 1]));
   pb.perm = tab.size();
   SPI_TRY(c->cg_buf[8].ensure(tab.size() * sizeof(int2) + (size_t)std::max(pb.nvox, 1ll) * sizeof(int)));
-  SPI_TRY(c->cg_buf[9].ensure(2 * (size_t)n * n * n * sizeof(double)));
   SPI_CUDA(cudaMemcpyAsync(c->cg_buf[8].p, tab.data(), tab.size() * sizeof(int2), cudaMemcpyHostToDevice, c->stream));
   const int2* d = c->cg_buf[8].as<int2>();
   cg_perm_kernel<<<(nbox + 7) / 8, 256, 0, c->stream>>>(d, reinterpret_cast<const int*>(d + box0), n, bx, by, nbox,
@@ -1003,6 +1006,18 @@ static int cg_lines(spi_ctx* c, CgProblem& pb) {
   SPI_TRY(check_kernel("cg_perm_kernel"));
   c->count();
   return 0;
+}
+
+// cg_buf[9] = room for the two layouts of the volume, 2 n^3 doubles; they only
+// make the projector's reads contiguous, so it does without where there is no room
+// (SPI_CG_LAYOUTS=0: never).  An iteration of 1,000 directions at 128^3 takes 6.0 ms
+// with them and 9.0 without, of 200 at 256^3 20.2 and 19.9.
+static void cg_layouts(spi_ctx* c, int n) {
+  const char* s = getenv("SPI_CG_LAYOUTS");
+  if ((s && atoi(s) == 0) || c->cg_buf[9].ensure(2 * (size_t)n * n * n * sizeof(double)) != 0) {
+    c->cg_buf[9].release();
+    cudaGetLastError();   // the failed allocation's
+  }
 }
 
 // A then A^T (BCKE += A^T A BCKP) chunk by chunk through PROJT tables
@@ -1022,8 +1037,9 @@ static int launch_normal_projt(spi_ctx* c, const CgProblem& pb, const double* x,
   static std::atomic<unsigned long long> attr_set{0};
   const unsigned long long bit = 1ull << (c->device & 63);
   if (!(attr_set.load() & bit)) {
-    cudaFuncSetAttribute(prjcq_projt_kernel<WIDE, WT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kProjSmem);
-    cudaFuncSetAttribute(prjcq_projt_kernel<WIDE, WT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kProjSmem);
+    for (auto kern : {prjcq_projt_kernel<WIDE, WT, false, true>, prjcq_projt_kernel<WIDE, WT, true, true>,
+                      prjcq_projt_kernel<WIDE, WT, false, false>, prjcq_projt_kernel<WIDE, WT, true, false>})
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kProjSmem);
     attr_set.fetch_or(bit);
   }
   const int C = mixed_bands(n, WIDE);
@@ -1032,18 +1048,21 @@ static int launch_normal_projt(spi_ctx* c, const CgProblem& pb, const double* x,
   const size_t smem = (size_t)(C == 1 ? n : (n + C - 1) / C + 2) * stride * (WIDE ? 8 : 4);
   double* const layouts = c->cg_buf[9].as<double>();
   const int2* const lines = c->cg_buf[8].as<int2>();
-  cg_layout_kernel<<<dim3((n + 31) / 32, (n + 31) / 32, 2 * n), dim3(32, 8), 0, c->stream>>>(x, n, layouts);
-  SPI_TRY(check_kernel("cg_layout_kernel"));
-  c->count();
+  if (layouts) {
+    cg_layout_kernel<<<dim3((n + 31) / 32, (n + 31) / 32, 2 * n), dim3(32, 8), 0, c->stream>>>(x, n, layouts);
+    SPI_TRY(check_kernel("cg_layout_kernel"));
+    c->count();
+  }
   for (int k0 = 0; k0 < nang; k0 += K) {
     const int kc = std::min(K, nang - k0);
     auto launch = [&](auto kern, int threads) {
-      kern<<<kc * C, threads, smem, c->stream>>>(layouts, lines, lines + (size_t)n * n, pb.ngroups, dms, lb, k0, n,
-                                                 stride, pb.ldp, C, maxabs, mcap, projt);
+      kern<<<kc * C, threads, smem, c->stream>>>(layouts ? layouts : x, lines, lines + (size_t)n * n, pb.ngroups, dms, lb,
+                                                 k0, n, stride, pb.ldp, C, maxabs, mcap, projt);
     };
     // one CTA per SM above half of its shared memory: twice the warps then
-    if (C == 1) launch(prjcq_projt_kernel<WIDE, WT, false>, smem > kProjSmem / 2 ? 1024 : 512);
-    else launch(prjcq_projt_kernel<WIDE, WT, true>, 512);
+    const int threads = C == 1 && smem > kProjSmem / 2 ? 1024 : 512;
+    if (layouts) launch(C == 1 ? prjcq_projt_kernel<WIDE, WT, false, true> : prjcq_projt_kernel<WIDE, WT, true, true>, threads);
+    else launch(C == 1 ? prjcq_projt_kernel<WIDE, WT, false, false> : prjcq_projt_kernel<WIDE, WT, true, false>, threads);
     SPI_TRY(check_kernel("prjcq_projt_kernel"));
     c->count();
     SPI_TRY((launch_backproject_projt<double, WT>(c, pb, out, projt, dms, k0, k0, k0 + kc)));
@@ -1529,6 +1548,7 @@ static int bpcg_run(spi_ctx* c, const float* projs, int n, int nang, const float
   SPI_TRY(c->cg_buf[6].ensure(3 * vb));
   if (mixed) SPI_TRY(cg_lines(c, pb));
   SPI_TRY(c->cg_buf[7].ensure(sizeof(CgScal) + 64 + (size_t)nang * sizeof(int)));
+  if (mixed) cg_layouts(c, n);
   T* cb = c->cg_buf[4].as<T>();
   T* pj = c->cg_buf[5].as<T>();
   float* pj32 = (mixed || fbs) ? c->cg_buf[5].as<float>()

@@ -41,6 +41,52 @@ def test_mixed_operators_match_fp64(ctx, monkeypatch, n, ri, bands, prec, tol):
     assert np.abs(v - ref).max() <= tol * np.abs(ref).max()
 
 
+def _solve_case(n, m):
+    g = np.random.default_rng(n)
+    ang = np.stack([g.uniform(0, 360, m), np.degrees(np.arccos(g.uniform(-1, 1, m))), g.uniform(0, 360, m)], 1).astype(np.float32)
+    return g.standard_normal((m, n, n)).astype(np.float32), ang
+
+
+@pytest.mark.parametrize("n,bands", [(11, None), (33, None), (66, "4"), (130, None)])
+def test_projector_without_layouts(ctx, monkeypatch, n, bands):
+    """The projector reading the volume itself sums the same integers as from the
+    layouts.  The solves' dot products are FP64 sums in any order, 1e-13 of the vectors, and the
+    volumes are rounded to FP32: equal to one last bit, 1.2e-7 of the largest voxel."""
+    if bands:
+        monkeypatch.setenv("SPI_CG_BANDS", bands)
+    img, ang = _solve_case(n, 40)
+    kw = dict(errm=1e-30, chim=0.0, maxit=2, mode=1, lam=0.5, ctx=ctx, fp64="mixed64")
+    ref, _ = ops.bpcg(img, ang, n // 2 - 3.0, **kw)
+    monkeypatch.setenv("SPI_CG_LAYOUTS", "0")
+    v, _ = ops.bpcg(img, ang, n // 2 - 3.0, **kw)
+    assert np.abs(v - ref).max() <= 1.2e-7 * np.abs(ref).max()
+
+
+def test_solve_without_room_for_layouts():
+    """With room for everything but the layouts (268 MB at 256^3), a solve runs without
+    them, as it did before it had them."""
+    import torch
+    n = 256
+    img, ang = _solve_case(n, 8)
+    kw = dict(errm=1e-30, chim=0.0, maxit=1, mode=1, lam=0.5)
+    c = ops.Context(0)
+    try:
+        ref, _ = ops.bpcg(img, ang, ctx=c, **kw)
+        need = c.device_bytes   # with the layouts
+    finally:
+        c.close()
+    c = ops.Context(0)
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - need + (134 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        v, _ = ops.bpcg(img, ang, ctx=c, **kw)
+    finally:
+        c.close()
+        del fill
+        torch.cuda.empty_cache()
+    assert np.abs(v - ref).max() <= 1.2e-7 * np.abs(ref).max()
+
+
 @pytest.mark.parametrize("prec", ["mixed64", "mixed", "fast"])
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_mixed_angle_not_finite(ctx, bad, prec):
