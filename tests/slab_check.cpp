@@ -1,25 +1,27 @@
-// CPU check of the column insertion's geometry (spider_b200/csrc/slab_geom.h):
-// for each box size and rotation the taps that the columns of every tile find
-// are compared, voxel by voxel, with ONELINE's own walk over the pixels
-// (restated here from oneline.f:38-200).
+// CPU check of the column insertion's and the extraction's geometry
+// (spider_b200/csrc/slab_geom.h).
 //
-//   slab_check NX SEED COUNT   ->  one line per rotation:
-//   kind banks max_rows max_pixels taps_direct taps_columns bad
+//   slab_check NX SEED COUNT   ->  two lines per rotation:
+//   kind banks columns max_rows max_pixels taps_direct taps_columns bad
+// compares, voxel by voxel, the taps that the columns of every tile find with
+// ONELINE's own walk over the pixels (restated here from oneline.f:38-200).  The
+// columns are walked in the blocks of slab_gather: `columns` = 2 (shallow slices in
+// FP32) and 1 (steep slices, and all in FP64; both lines of a steep one).  `bad` counts taps that only one side has or whose three table
+// entries differ, taps outside their column's voxel range, look-ups beyond the
+// table in shared memory, and tiles over the capacity.
+//
 //   slab_check extract NX SEED COUNT   ->  bad
 // counts look-ups and voxels of the extraction's pixels that are out of range, and
 // matrices with an element or angle that is not finite which are taken for a
 // rotation's.
-//
-// `bad` of the first form counts voxels whose set of (pixel, weight bits) differs, taps outside
-// their column's voxel range, tiles over the capacity, and pixel rows or spans
-// that do not cover a tap.
+#include <algorithm>
 #include <cstdint>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
-#include <map>
+#include <iterator>
 #include <random>
-#include <utility>
+#include <tuple>
 #include <vector>
 
 #include "../spider_b200/csrc/slab_geom.h"
@@ -28,12 +30,17 @@ using namespace spi;
 
 static std::vector<float> g_tab;
 static float g_fltb;
-static const int kLast = 3331;
+static const int kLast = kSlabTab - 1;
 
+// the kernel's look-up, and ONELINE's with Fortran's NINT
 static float tap(float c, int k) { return g_tab[slab_tab_index(c, k, g_fltb, kLast)]; }
+static float tap_nint(float c, int k) {
+  const float v = fabsf(c - (float)k) * g_fltb, f = floorf(v);
+  return g_tab[(int)f + (v - f >= 0.5f ? 1 : 0)];
+}
 
-// key of a tap: voxel and pixel (of the full disc), value: bits of the weight
-typedef std::map<std::pair<long long, int>, std::vector<uint32_t>> Taps;
+// a tap: voxel, pixel of the full disc, bits of its weights along x, y and z
+typedef std::tuple<long long, int, uint32_t, uint32_t, uint32_t> Tap;
 
 static long long vox(int x, int y, int z, int nx) {
   const int N = 2 * nx;
@@ -41,17 +48,15 @@ static long long vox(int x, int y, int z, int nx) {
   return ((long long)iz * N + iy) * (nx + 1) + x;
 }
 
-static uint32_t wbits(float wx, float wy, float wz) {
-  const float w = wx * (wy * wz);
+static uint32_t bits(float w) {
   uint32_t b;
   memcpy(&b, &w, 4);
   return b;
 }
 
 // ONELINE over the half disc; pixel id of the canonical pixel and its mate
-static long long direct(const float* dm, int nx, Taps& t) {
+static void direct(const float* dm, int nx, std::vector<Tap>& t) {
   const int N = 2 * nx, W = 2 * nx + 1;
-  long long n = 0;
   for (int J = -nx + 1; J <= nx; ++J)
     for (int I = 0; I <= nx; ++I) {
       if (I * I + J * J >= nx * nx || (I == 0 && J < 0)) continue;
@@ -69,16 +74,14 @@ static long long direct(const float* dm, int nx, Taps& t) {
         for (int ly = -2; ly <= 2; ++ly)
           for (int lx = -2; lx <= 2; ++lx) {
             const int x = k[0] + lx, y = k[1] + ly, z = k[2] + lz;
-            const float wx = tap(c[0], x), wy = tap(c[1], y), wz = tap(c[2], z);
+            const float wx = tap_nint(c[0], x), wy = tap_nint(c[1], y), wz = tap_nint(c[2], z);
             if (wx * (wy * wz) == 0.0f) continue;
             // pixel that lies where the tap lands: the canonical one, or its mate for a reflected tap
             const int sg = x < 0 ? -s : s;
             const int id = (sg * J + nx) * W + sg * I + nx;
-            t[{x < 0 ? vox(-x, -y, -z, nx) : vox(x, y, z, nx), id}].push_back(wbits(wx, wy, wz));
-            ++n;
+            t.push_back({x < 0 ? vox(-x, -y, -z, nx) : vox(x, y, z, nx), id, bits(wx), bits(wy), bits(wz)});
           }
     }
-  return n;
 }
 
 // CANG in REAL (cang.f:44-81)
@@ -151,98 +154,92 @@ int main(int argc, char** argv) {
   g_tab.assign(5000, 0.0f);
   for (int i = 0; i < 5000; ++i)
     if ((float)i / g_fltb <= 1.8f) g_tab[i] = 1.0f + (float)(5000 - i) * 1.37e-4f;
-  std::uniform_real_distribution<double> U(0.0, 1.0);
+  std::uniform_real_distribution<float> U(0.0f, 1.0f);
+  const float mag = 54.735610f;   // acos(1 / sqrt(3))
   for (int q = 0; q < count; ++q) {
-    double ps = 2 * M_PI * U(rng), th = acos(1 - 2 * U(rng)), ph = 2 * M_PI * U(rng);
+    float d[3] = {360.0f * U(rng), 57.29578f * std::acos(1.0f - 2.0f * U(rng)), 360.0f * U(rng)};
     // the rotations where the geometry degenerates come first: axes, diagonals, planes of 45 degrees
-    const double sp[12][3] = {{0, 0, 0}, {0, M_PI / 2, 0}, {0, M_PI / 2, M_PI / 2}, {M_PI / 4, 0, 0},
-                              {0, M_PI / 4, 0}, {M_PI / 4, acos(1 / sqrt(3.0)), M_PI / 4}, {0, M_PI, 0},
-                              {M_PI / 2, M_PI / 2, M_PI / 4}, {0.3, M_PI / 2, M_PI / 4}, {M_PI, acos(1 / sqrt(3.0)), -M_PI / 4},
-                              {0, acos(1 / sqrt(3.0)), M_PI / 4}, {1.1, M_PI / 4, M_PI / 2}};
-    if (q < 12) { ps = sp[q][0]; th = sp[q][1]; ph = sp[q][2]; }
-    const double cp = cos(ps), s_p = sin(ps), ct = cos(th), st = sin(th), cf = cos(ph), sf = sin(ph);
-    const float dm[6] = {(float)(cf * ct * cp - sf * s_p), (float)(sf * ct * cp + cf * s_p), (float)(-st * cp),
-                         (float)(-cf * ct * s_p - sf * cp), (float)(-sf * ct * s_p + cf * cp), (float)(st * s_p)};
-    Taps A, B;
-    long long na = direct(dm, nx, A), nb = 0, bad = 0;
+    const float sp[12][3] = {{0, 0, 0}, {0, 90, 0}, {0, 90, 90}, {45, 0, 0}, {0, 45, 0}, {45, mag, 45}, {0, 180, 0},
+                             {90, 90, 45}, {17.2f, 90, 45}, {180, mag, -45}, {0, mag, 45}, {63, 45, 90}};
+    if (q < 12) memcpy(d, sp[q], sizeof(d));
+    float dm[6];
+    euler(d[0], d[1], d[2], dm);
+    std::vector<Tap> A, B;
+    direct(dm, nx, A);
+    std::sort(A.begin(), A.end());
     SlabFrame f;
-    int rows = 0, pixels = 0, banks = 0;
     if (!slab_frame(dm, f)) { printf("noframe\n"); continue; }
-    banks = slab_banks(f);
-    const int nu = banks == 2 ? 2 : 1;   // columns along u of a thread's block
-    const int W = 2 * nx + 1;
+    const int banks = slab_banks(f), W = 2 * nx + 1;
     const int ntu = f.d == 0 ? (2 * nx + kSlabTile - 1) / kSlabTile : (nx + kSlabTile - 1) / kSlabTile;
     const int ntv = (2 * nx + kSlabTile - 1) / kSlabTile;
-    for (int tv = 0; tv < ntv; ++tv)
-      for (int tu = 0; tu < ntu; ++tu) {
-        const int u0 = (f.d == 0 ? -nx : 0) + kSlabTile * tu, v0 = -nx + kSlabTile * tv;
-        if (!slab_tile_live(f, u0, v0, nx)) continue;
-        int jlo, nr;
-        slab_tile_rows(f, u0, v0, nx, jlo, nr);
-        std::vector<int> lo(nr), hi(nr);
-        int np = 0;
-        for (int r = 0; r < nr; ++r) {
-          slab_tile_span(f, u0, v0, nx, jlo + r, lo[r], hi[r]);
-          np += hi[r] >= lo[r] ? hi[r] - lo[r] + 1 : 0;
-        }
-        if (nr > rows) rows = nr;
-        if (np > pixels) pixels = np;
-        if (nr >= kSlabRows || np > kSlabPix) ++bad;
-        for (int du = 0; du < kSlabTile; du += nu)
-          for (int dv = 0; dv < kSlabTile; dv += 2) {   // a block of columns at a time, as the kernel's threads take them
-            int r0, r1;
-            const float u = (float)(u0 + du), v = (float)(v0 + dv);
-            slab_block_rows(f, u, v, nu, 2, jlo, nr, r0, r1);
-            for (int r = r0; r <= r1; ++r) {
-              float fl, fh;
-              slab_span(f, u + 0.5f * (nu - 1), v + 0.5f, kSlabR + 0.5f * (nu - 1), kSlabR + 0.5f, jlo + r, fl, fh);
-              const int i0 = slab_ceil(fmaxf(fl, (float)lo[r])), i1 = slab_floor(fminf(fh, (float)hi[r]));
-              for (int I = i0; I <= i1; ++I) {
-                const SlabPix p = slab_pixel(f, I, jlo + r);
-                if (!slab_inside(f, p, I, jlo + r, nx)) continue;
-                const int au = f.d == 0 ? 1 : 0, av = f.d == 2 ? 1 : 2, aw = f.d;
-                float pos[3];
-                pos[au] = p.u;
-                pos[av] = p.v;
-                pos[aw] = p.w;
-                for (int c = 0; c < 2 * nu; ++c) {
-                  int k[3];
-                  k[au] = u0 + du + c / 2;
-                  k[av] = v0 + dv + c % 2;
-                  // the kernel's table has no bound on the index
-                  if (slab_tab_index(p.u, k[au], g_fltb, 9999) >= kSlabTab || slab_tab_index(p.v, k[av], g_fltb, 9999) >= kSlabTab) ++bad;
-                  const int base = slab_col_base(f, (float)k[au], (float)k[av]);
-                  for (int l = 0; l < 4; ++l) {
-                    k[aw] = slab_first(p.w) + l;
-                    const float wx = tap(pos[0], k[0]), wy = tap(pos[1], k[1]), wz = tap(pos[2], k[2]);
-                    if (wx * (wy * wz) == 0.0f) continue;
-                    if (k[0] < 0 || (k[0] == 0 && !p.canon)) continue;
-                    // the residue must give the voxel back
-                    const int off = slab_residue(k[aw], banks) - slab_residue(base, banks);
-                    if (base + (off < 0 ? off + 4 * banks : off) != k[aw]) ++bad;
-                    B[{vox(k[0], k[1], k[2], nx), (jlo + r + nx) * W + I + nx}].push_back(wbits(wx, wy, wz));
-                    ++nb;
+    for (int form = 0; form < 2; ++form) {
+      const int nc = form == 0 && banks == 2 ? 2 : 1;   // columns along v of a thread's block
+      long long bad = 0;
+      int rows = 0, pixels = 0;
+      B.clear();
+      for (int tv = 0; tv < ntv; ++tv)
+        for (int tu = 0; tu < ntu; ++tu) {
+          const int u0 = (f.d == 0 ? -nx : 0) + kSlabTile * tu, v0 = -nx + kSlabTile * tv;
+          if (!slab_tile_live(f, u0, v0, nx)) continue;
+          int jlo, nr;
+          slab_tile_rows(f, u0, v0, nx, jlo, nr);
+          std::vector<int> lo(nr), hi(nr);
+          int np = 0;
+          for (int r = 0; r < nr; ++r) {
+            slab_tile_span(f, u0, v0, nx, jlo + r, lo[r], hi[r]);
+            np += hi[r] >= lo[r] ? hi[r] - lo[r] + 1 : 0;
+          }
+          if (nr > rows) rows = nr;
+          if (np > pixels) pixels = np;
+          if (nr >= kSlabRows || np > kSlabPix) ++bad;
+          for (int du = 0; du < kSlabTile; ++du)
+            for (int dv = 0; dv < kSlabTile; dv += nc) {
+              int r0, r1;
+              const float u = (float)(u0 + du), v = (float)(v0 + dv);
+              slab_block_rows(f, u, v, 1, nc, jlo, nr, r0, r1);
+              for (int r = r0; r <= r1; ++r) {
+                float fl, fh;
+                slab_span(f, u, v + 0.5f * (nc - 1), kSlabR, kSlabR + 0.5f * (nc - 1), jlo + r, fl, fh);
+                const int i0 = slab_ceil(fmaxf(fl, (float)lo[r])), i1 = slab_floor(fminf(fh, (float)hi[r]));
+                for (int I = i0; I <= i1; ++I) {
+                  const SlabPix p = slab_pixel(f, I, jlo + r);
+                  if (!slab_inside(f, p, I, jlo + r, nx)) continue;
+                  const int au = f.d == 0 ? 1 : 0, av = f.d == 2 ? 1 : 2, aw = f.d;
+                  float pos[3];
+                  pos[au] = p.u;
+                  pos[av] = p.v;
+                  pos[aw] = p.w;
+                  for (int c = 0; c < nc; ++c) {
+                    int k[3];
+                    k[au] = u0 + du;
+                    k[av] = v0 + dv + c;
+                    // the kernel's table has no bound on the index
+                    if (slab_tab_index(p.u, k[au], g_fltb, 9999) >= kSlabTab || slab_tab_index(p.v, k[av], g_fltb, 9999) >= kSlabTab) ++bad;
+                    const int base = slab_col_base(f, (float)k[au], (float)k[av]);
+                    for (int l = 0; l < 4; ++l) {
+                      k[aw] = slab_first(p.w) + l;
+                      const float wx = tap(pos[0], k[0]), wy = tap(pos[1], k[1]), wz = tap(pos[2], k[2]);
+                      if (wx * (wy * wz) == 0.0f) continue;
+                      if (k[0] < 0 || (k[0] == 0 && !p.canon)) continue;
+                      // the residue must give the voxel back
+                      const int off = slab_residue(k[aw], banks) - slab_residue(base, banks);
+                      if (base + (off < 0 ? off + 4 * banks : off) != k[aw]) ++bad;
+                      B.push_back({vox(k[0], k[1], k[2], nx), (jlo + r + nx) * W + I + nx, bits(wx), bits(wy), bits(wz)});
+                    }
                   }
                 }
               }
             }
-          }
-      }
-    // the origin's reflected taps (it is its own mate)
-    const int id0 = nx * W + nx;
-    for (int x = 1; x <= 1; ++x)
-      for (int y = -1; y <= 1; ++y)
-        for (int z = -1; z <= 1; ++z) {
-          B[{vox(x, -y, -z, nx), id0}].push_back(wbits(tap(0, x), tap(0, y), tap(0, z)));
-          ++nb;
         }
-    for (auto& e : A) {
-      auto it = B.find(e.first);
-      if (it == B.end() || it->second != e.second) ++bad;
+      // the origin's reflected taps (it is its own mate)
+      for (int y = -1; y <= 1; ++y)
+        for (int z = -1; z <= 1; ++z) B.push_back({vox(1, -y, -z, nx), nx * W + nx, bits(tap(0, 1)), bits(tap(0, y)), bits(tap(0, z))});
+      std::sort(B.begin(), B.end());
+      std::vector<Tap> only;
+      std::set_symmetric_difference(A.begin(), A.end(), B.begin(), B.end(), std::back_inserter(only));
+      bad += (long long)only.size();
+      printf("%d %d %d %d %d %zu %zu %lld\n", f.d, banks, nc, rows, pixels, A.size(), B.size(), bad);
     }
-    for (auto& e : B)
-      if (!A.count(e.first)) ++bad;
-    printf("%d %d %d %d %lld %lld %lld\n", f.d, banks, rows, pixels, na, nb, bad);
   }
   return 0;
 }
