@@ -164,24 +164,20 @@ def test_bp3f_config1_full(ctx, orc):
 
 def test_insert_kernels_agree(ctx, orc):
     """The tile-privatised insertion and the direct per-tap insertion add the
-    same taps; they differ only in FP32 summation order.  So do the x4
-    kernel's row-by-row, column-by-column and per-slice insertion orders."""
+    same taps; they differ in the order of the FP32 products and sums.  So do the
+    five-lane, the column (x4) and the fixed-point tile kernels."""
     nx, nimg = 48, 300
     _, pr, ang = _case(nx, nimg, 61)
     # include orientations that put the x = 0 flip line inside many tiles
     ang[:40, 1] = 90.0
     out, grids = {}, {}
-    for mode in ("direct", "tile", "xlane", "x4", "tilefx", "x4:rows", "x4:cols"):
-        kernel, _, order = mode.partition(":")
-        os.environ["SPI_INSERT"] = kernel
-        if order:
-            os.environ["SPI_INSERT_ORDER"] = order
+    for mode in ("direct", "tile", "xlane", "x4", "tilefx"):
+        os.environ["SPI_INSERT"] = mode
         try:
             out[mode] = ops.bp3f(pr, ang, ctx=ctx)
             grids[mode] = ops.bp3f_partial(pr, ang, ctx=ctx)
         finally:
             del os.environ["SPI_INSERT"]
-            os.environ.pop("SPI_INSERT_ORDER", None)
     ref = orc.bp3f(pr, ang, prec=1, nthreads=1)
     for mode, v in out.items():
         assert synth.rel_l2(v, out["direct"]) <= 2e-6, mode
@@ -212,12 +208,11 @@ def test_rb3f_rb32f_match_oracle(ctx, orc):
     assert synth.rel_l2(z, ops.bp3f(pr, ang, ctx=ctx)) <= 2e-6
 
 
-@pytest.mark.parametrize("mode", ["one_launch", "one_launch:cols", "one_launch:own", "concurrent", "in_turn"])
+@pytest.mark.parametrize("mode", ["one_launch", "one_launch:own", "concurrent", "in_turn"])
 def test_bp32f_multiclass(orc, mode):
     """Several classes of different box sizes (one odd, two equal) reconstructed
     from one image stream: all classes in one insertion launch per round
-    (spi_bp_insert_multi; also with every slice inserted column by column),
-    or one context per class inserted concurrently from one host thread
+    (spi_bp_insert_multi; also with the own R2C where it applies), or one context per class inserted concurrently from one host thread
     each, or in turn."""
     classes, refs = [], []
     for k, (nx, nimg) in enumerate(((24, 120), (32, 200), (41, 150), (32, 90))):
@@ -226,14 +221,11 @@ def test_bp32f_multiclass(orc, mode):
         classes.append((pr, ang, half))
         refs.append(orc.bp32f(pr, ang, half, prec=0, nthreads=1))
     mode, _, opt = mode.partition(":")
-    if opt == "cols":
-        os.environ["SPI_INSERT_ORDER"] = opt
-    elif opt == "own":   # the own R2C for the power-of-two padded box (32 -> 64), cuFFT for the others
+    if opt == "own":   # the own R2C for the power-of-two padded box (32 -> 64), cuFFT for the others
         os.environ["SPI_FFT"] = opt
     try:
         out = ops.bp32f_multiclass(classes, one_launch=mode == "one_launch", concurrent=mode == "concurrent")
     finally:
-        os.environ.pop("SPI_INSERT_ORDER", None)
         os.environ.pop("SPI_FFT", None)
     for got, ref in zip(out, refs):
         for a, b in zip(got, ref):

@@ -19,7 +19,8 @@ def _angles(n, seed):
     return ang
 
 
-@pytest.mark.parametrize("nx,nimg", [(8, 9), (15, 40), (16, 1), (17, 40), (33, 60), (40, 700)])
+# rows of tiles split into parts (a launch of few slices) and whole ones (1,000 at 33^3)
+@pytest.mark.parametrize("nx,nimg", [(8, 9), (15, 40), (16, 1), (17, 40), (33, 60), (33, 1000), (40, 700)])
 def test_columns_match_oracle_grids(ctx, orc, nx, nimg):
     """X and W grids within 2e-6 of the FP64 sums: the products' three roundings
     (1e-7) and the random walk of at most a few hundred FP32 additions of 6e-8
@@ -31,6 +32,60 @@ def test_columns_match_oracle_grids(ctx, orc, nx, nimg):
     xr, wr = orc.bp3f_partial(imgs, ang, prec=1, nthreads=1)
     assert synth.rel_l2(w, wr) <= 2e-6
     assert synth.rel_l2(x, np.stack([xr.real, xr.imag], -1)) <= 2e-6
+
+
+def _frame(ang):
+    """Dominant axis of a slice's normal and the banks of its columns (slab_frame, slab_banks)."""
+    psi, th, phi = np.radians(np.asarray(ang, np.float64))
+    n = np.array([np.sin(th) * np.cos(phi), np.sin(th) * np.sin(phi), np.cos(th)])
+    d = int(np.argmax(np.abs(n)))
+    rise = sum(abs(n[a] / n[d]) for a in range(3) if a != d)   # |SU| + |SV|
+    return d, 2 if 1.81 * (1 + rise) + 0.01 <= 4.0 else 3
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("banks", [2, 3])
+def test_columns_by_frame(ctx, orc, axis, banks, bf16):
+    """Slices of one dominant axis and one bank count at a time, FP32 and BF16 spectra:
+    W within 2e-6 of the FP64 sums either way; X 2e-6 in FP32, in BF16 2^-9 (half a unit
+    of its 8 bits) for every value."""
+    nx = 24
+    rng = np.random.default_rng(10 * axis + banks)
+    ang = synth.so3_angles(900, rng)
+    ang = ang[[_frame(a) == (axis, banks) for a in ang]][:40]
+    assert len(ang) == 40
+    imgs = rng.standard_normal((40, nx, nx)).astype(np.float32)
+    ctx.bp_open(nx, 1, bf16=bf16)
+    try:
+        ctx.bp_insert(imgs, ang)
+        x, w = ctx.bp_partial_out(0)
+    finally:
+        ctx.bp_close()
+    xr, wr = orc.bp3f_partial(imgs, ang, prec=1, nthreads=1)
+    assert synth.rel_l2(w, wr) <= 2e-6
+    assert synth.rel_l2(x, np.stack([xr.real, xr.imag], -1)) <= (2.0 ** -9 if bf16 else 2e-6)
+
+
+def test_columns_two_classes_in_turn(orc):
+    """Classes of two box sizes in one launch, whose tables a CTA loads as it meets
+    them: each class's grid is that of its own insertion."""
+    rng = np.random.default_rng(31)
+    cs = [ops.Context(0), ops.Context(0)]
+    try:
+        data = []
+        for c, nx, n in zip(cs, (20, 33), (300, 200)):
+            c.bp_open(nx, 1)
+            data.append((rng.standard_normal((n, nx, nx)).astype(np.float32), synth.so3_angles(n, rng)))
+        ops.bp_insert_multi(cs, [(imgs, ang, None) for imgs, ang in data])
+        for c, (imgs, ang) in zip(cs, data):
+            x, w = c.bp_partial_out(0)
+            xr, wr = orc.bp3f_partial(imgs, ang, prec=1, nthreads=1)
+            assert synth.rel_l2(w, wr) <= 2e-6
+            assert synth.rel_l2(x, np.stack([xr.real, xr.imag], -1)) <= 2e-6
+    finally:
+        for c in cs:
+            c.close()
 
 
 def test_columns_not_finite(ctx):
