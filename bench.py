@@ -467,7 +467,7 @@ def fourier_cg_measure(ctx, projs, ang, K, lam=1e-3, check_images=1000, check_it
     """The differentiable reconstruction on the FourierSlice pair (E = central
     slice extraction, E^T = ONELINE's insertion without weights): CG on
     (E^T E + lam I) x = E^T b from the staged image spectra, one iteration
-    (the fused normal operator + FP64 dot products) replayed as a CUDA graph
+    (the normal operator + FP64 dot products) replayed as a CUDA graph
     against the same iteration launched op by op.  rel_err_vs_fp64_oracle: the
     graph-captured CG after `check_iters` iterations against an FP64 CG on
     the oracle's pair, on the first `check_images` images."""

@@ -2641,7 +2641,7 @@ static int bp_insert_impl(spi_ctx* c, const float* imgs, int nimg, const float* 
 // runs on the first context's stream: while the call runs, the other
 // classes' contexts use that stream (their own are idle and restored after).
 namespace {
-constexpr int kMcMaxSizes = 8;
+constexpr int kMcMaxSizes = 8;   // distinct boxes that the entry point takes in one call (spider_b200.h)
 struct StreamSwap {
   std::vector<spi_ctx*> ctxs;
   std::vector<cudaStream_t> saved;

@@ -4,15 +4,16 @@
 // Operators (voxel runs from PREPCUB_S, prepcub_s.f:54-111):
 //   A   = PRJCQ_N (prjcq.f:48-82): every sphere voxel splats bilinearly into
 //         the projection.  One CTA per projection keeps the image in shared
-//         memory (n <= 224) and walks whole runs with the reference's
+//         memory (200 KB of it) and walks whole runs with the reference's
 //         sequential XB = XB + DM(1) accumulation, so sample positions are
 //         bit-identical; shared-memory atomics accumulate.
 //   A^T = BCKPJ_LIN (bckpj.f:59-94, SP_MP branch): every sphere voxel
 //         gathers from each projection through the PROJT difference table
 //         (bpcg.f:732-742), computed on the fly from four pixels with the
-//         same float operations.  One thread per voxel sums the projections
-//         in image order, the order of the reference's image loop, so the
-//         back-projection is bit-identical to the CPU form.
+//         same float operations (the mixed modes make the table first).
+//         One thread per voxel sums the projections in image order, the order
+//         of the reference's image loop, so the back-projection is
+//         bit-identical to the CPU form.
 // CG scalars (DELSQ, AKDEN, P, Q) are FP64 device scalars; the vectors and
 // projections are FP64 by default and FP32 (the reference's REAL) on request.
 // One CG iteration is a fixed kernel sequence captured once as a CUDA graph.

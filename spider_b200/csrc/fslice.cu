@@ -16,11 +16,11 @@
 // Grid: complex float2 [2nx][2nx][nx+1] (i fastest, Fortran X(0:NX,N,N)).
 // Slices: float2 [nslice][2nx][nx+1] in the layout and sign of the staged
 // spectra the back-projection inserts (cuFFT R2C of the padded, shifted
-// image; ONELINE's BI is its conjugate).  Every tap -- voxel, table weight,
-// Hermitian flip (x < 0), reflected point (oneline.f:118-150) -- is computed
-// that of the back-projection's insertion: E is fs_extract.cuh, E^T the column
-// insertion of slab.cuh; the normal operators without a buffer take four lanes
-// per pixel over the nonzero window of the table.
+// image; ONELINE's BI is its conjugate).  Every tap (voxel, table weight,
+// Hermitian flip for x < 0, reflected point, oneline.f:118-150) is that of the
+// back-projection's insertion.  E is fs_extract.cuh, E^T the column insertion of
+// slab.cuh; the normal operators without a buffer take four lanes per pixel over
+// the nonzero window of the table.
 #include <algorithm>
 #include <atomic>
 #include <cmath>

@@ -84,8 +84,8 @@ __device__ __forceinline__ void slab_red64(void* grid, size_t i, double re, doub
 
 constexpr int kSlabMaxClass = 16;
 constexpr int kSlabThreads = kSlabTile * kSlabTile / 2;   // consumers: two columns each, neighbours along v
-constexpr int kSlabBlocks = 4;                            // CTAs per SM (96 registers, 50 KB each)
-constexpr int kSlabBlocks64 = 3;                          // the same with FP64 sums (128 registers, 50-60 KB)
+constexpr int kSlabBlocks = 4;                            // CTAs per SM (96 registers, 54 KB each)
+constexpr int kSlabBlocks64 = 3;                          // the same with FP64 sums (128 registers, 48-59 KB)
 
 struct SlabClass {
   const void* spec;            // spectra of the class's images in this launch
@@ -122,6 +122,9 @@ struct SlabSmem {
   typename F::Raw raw[2][kSlabPix];   // slice values
   float tab[kSlabTab];
 };
+// an SM's 228 KB hold kSlabBlocks (kSlabBlocks64) of them, with the kilobyte that each CTA takes besides
+static_assert(sizeof(SlabSmem<SlabBp>) <= (228 / kSlabBlocks - 1) * 1024, "four CTAs per SM");
+static_assert(sizeof(SlabSmem<SlabFs64d>) <= (228 / kSlabBlocks64 - 1) * 1024, "three CTAs per SM");
 
 __device__ __forceinline__ unsigned long long slab_pack(float a, float b) {
   unsigned long long r;

@@ -80,7 +80,8 @@ constexpr float kSlabR = 1.81f;
 constexpr int kSlabRows = 48, kSlabPix = 656;
 
 // Entries of a table kept in shared memory: a table kb_window4_ok accepts is
-// zero from floor(2 FLTB) - 1 = 3331 on.  Looking a pixel up for the columns
+// zero from floor(1.805 FLTB) = 3,007 on, which is also why columns within
+// kSlabR of a pixel hold all of its taps.  Looking a pixel up for the columns
 // of a block reaches distances of 1.81 + 1 and a rounding below 0.001, entry
 // 4,685, so with zeros up to there no index needs a bound.
 constexpr int kSlabTab = 4736;
