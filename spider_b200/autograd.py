@@ -169,14 +169,22 @@ class FourierSlicePlan:
     def _normal(self, grid, lam, out):
         """E^T (E grid) + lam grid through a slice buffer from torch's allocator: one per
         call, on the call's stream, so calls on several streams do not share it.  Where
-        there is no room for one, the form that keeps no slices runs instead."""
+        there is no room for one, and for small plans, the form that keeps no slices runs
+        instead (us without / with the buffer: 16^3 with 16, 256, 512 slices 29/59, 57/79, 97/101, in
+        FP64 29/62, 97/104, 165/131; 64^3 with 16, 32, 64 64/80, 101/95, 145/129; 96^3 with 16,
+        32 101/103, 160/137; 128^3 with 4 151/136)."""
         import ctypes
+        small = self.nx < 128 and self.nang <= 256 and self.nang * self.nx ** 2 <= 1 << 17
         fp64 = int(grid.dtype == torch.float64)
-        nb = ctypes.c_longlong()
-        ops.check(self._L.spi_fslice_normal_ws_bytes(self._h, fp64, ctypes.byref(nb)))
-        try:
-            ws = torch.empty(nb.value, dtype=torch.uint8, device=self.device)
-        except torch.OutOfMemoryError:
+        ws = None
+        if not small:
+            nb = ctypes.c_longlong()
+            ops.check(self._L.spi_fslice_normal_ws_bytes(self._h, fp64, ctypes.byref(nb)))
+            try:
+                ws = torch.empty(nb.value, dtype=torch.uint8, device=self.device)
+            except torch.OutOfMemoryError:
+                pass
+        if ws is None:
             one_pass = self._L.spi_fslice_normal64 if fp64 else self._L.spi_fslice_normal
             ops.check(one_pass(self._h, ctypes.c_void_p(grid.data_ptr()), float(lam), ctypes.c_void_p(out.data_ptr()),
                                self._stream()))

@@ -19,8 +19,8 @@
 // image; ONELINE's BI is its conjugate).  Every tap (voxel, table weight,
 // Hermitian flip for x < 0, reflected point, oneline.f:118-150) is that of the
 // back-projection's insertion.  E is fs_extract.cuh, E^T the column insertion of
-// slab.cuh; the normal operators without a buffer take four lanes per pixel over
-// the nonzero window of the table.
+// slab.cuh; E^T of few slices and the normal operators without a buffer take four
+// lanes per pixel over the nonzero window of the table.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -54,6 +54,8 @@ struct FsWin {
   float ty[4], tz[4];
 };
 
+// LS: lanes per x tap (the y/z weight of window position l lives in lane gl + l * LS).
+template <int LS = 1>
 __device__ __forceinline__ void fs_window(const SliceDesc& sd, int I, int J, int nx, const float* tab, float fltb,
                                           int q, int gl, FsWin& w) {
   const int N = 2 * nx, N2 = nx, LN2 = 2, NN4 = N * N / 4;
@@ -82,8 +84,8 @@ __device__ __forceinline__ void fs_window(const SliceDesc& sd, int I, int J, int
   const float tzq = fs_tap(tab, znew, w.zs + q, fltb);
 #pragma unroll
   for (int l = 0; l < 4; ++l) {
-    w.ty[l] = __shfl_sync(0xffffffffu, tyq, gl + l);
-    w.tz[l] = __shfl_sync(0xffffffffu, tzq, gl + l);
+    w.ty[l] = __shfl_sync(0xffffffffu, tyq, gl + l * LS);
+    w.tz[l] = __shfl_sync(0xffffffffu, tzq, gl + l * LS);
   }
   w.ok = ok && w.tx != 0.0f;
 }
@@ -143,6 +145,64 @@ __device__ __forceinline__ void fs_scatter(float2* __restrict__ X, const FsWin& 
       bool refl;
       const size_t v = fs_voxel(w, q, ly, lz, nx, refl);
       atomicAdd(X + v, fs_cmul(b, wg, refl));
+    }
+  }
+}
+
+// The same into an FP64 grid, the real (h = 0) or the imaginary part b of the value
+__device__ __forceinline__ void fs_scatter_part(double* __restrict__ X, const FsWin& w, int q, int h, int nx, double b) {
+  if (!w.ok) return;
+#pragma unroll
+  for (int lz = 0; lz < 4; ++lz) {
+    if (w.tz[lz] == 0.0f) continue;
+#pragma unroll
+    for (int ly = 0; ly < 4; ++ly) {
+      const float tyz = __fmul_rn(w.ty[ly], w.tz[lz]);
+      if (tyz == 0.0f) continue;
+      const float wg = __fmul_rn(w.tx, tyz);
+      if (wg == 0.0f) continue;
+      bool refl;
+      const size_t v = fs_voxel(w, q, ly, lz, nx, refl);
+      const double t = __dmul_rn(b, (double)wg);
+      atomicAdd(X + 2 * v + h, h && refl ? -t : t);
+    }
+  }
+}
+
+// E^T tap by tap, for plans too small for the columns (fs_small): a warp takes
+// one row J of one slice and adds every tap with a reduction of its own.  X += E^T
+// of the slices.  FP32: eight pixels at a time, four lanes per pixel.  FP64: four
+// pixels, eight lanes, so that one instruction adds both parts of four
+// consecutive voxels (64 contiguous bytes): 256 slices at 16^3 66 us, 91 with four lanes.
+template <bool D>
+__global__ void __launch_bounds__(256) fs_taps_kernel(const float2* __restrict__ in, void* __restrict__ out,
+                                                      const SliceDesc* __restrict__ slices, int nslices, int nx,
+                                                      const float* __restrict__ kbtab, float fltb) {
+  extern __shared__ float tab[];
+  for (int i = threadIdx.x; i < 5000; i += blockDim.x) tab[i] = kbtab[i];
+  __syncthreads();
+  constexpr int kLanes = D ? 8 : 4;
+  const int N = 2 * nx, NN4 = nx * nx;
+  const int lane = threadIdx.x & 31;
+  const int g = lane / kLanes, q = lane % kLanes / (kLanes / 4), h = lane & 1, gl = lane & ~(kLanes - 1);
+  const long long nitems = (long long)nslices * N;
+  const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+  for (long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < nitems;
+       item += warps) {
+    const SliceDesc sd = slices[item / N];
+    const int J = (int)(item % N) - nx + 1;
+    const float2* row = in + ((size_t)sd.img * N + (J >= 0 ? J : N + J)) * (size_t)(nx + 1);
+    for (int I0 = 0; I0 * I0 + J * J < NN4; I0 += 32 / kLanes) {   // warp-uniform
+      FsWin w;
+      fs_window<kLanes / 4>(sd, I0 + g, J, nx, tab, fltb, q, gl, w);
+      // BTQ = BI = conj(T), or conj(BI) = T for a flipped pixel
+      float2 b = make_float2(0.0f, 0.0f);
+      if (w.ok) {
+        const float2 t = row[I0 + g];
+        b = make_float2(t.x, w.flipped ? t.y : -t.y);
+      }
+      if (D) fs_scatter_part(static_cast<double*>(out), w, q, h, nx, (double)(h ? b.y : b.x));
+      else fs_scatter(static_cast<float2*>(out), w, q, nx, b);
     }
   }
 }
@@ -390,12 +450,33 @@ template <class F>
 int fs_insert(const spi_fslice_plan* p, const void* slices, void* grid, int first, int count, unsigned long long* work,
               cudaStream_t s);
 
+// Is E^T of the plan's slices faster tap by tap?  A column tile takes 10 to 20 us
+// from its fetch to its sums, whatever the launch (steep slices most); in small
+// boxes the reductions of few slices are over before.  us tap by tap / by columns,
+// FP32: 16^3 with 1, 64, 256, 512 slices 21/34, 26/45, 57/57, 84/72; 64^3 with 1,
+// 16, 64, 96 33/32, 39/57, 77/80, 100/98; 80^3 with 16, 64 52/63, 113/98; 96^3 with 1,
+// 8, 16 44/33, 50/61, 62/58.  FP64: 16^3 with 64, 256, 512 32/60, 66/83, 104/96; 32^3
+// with 1, 64, 128 34/31, 60/73, 93/88; 48^3 with 4, 16, 48 43/39, 53/55, 92/78; 64^3
+// with 1, 16, 32 52/35, 67/84, 95/91.
+bool fs_small(const spi_fslice_plan* p, bool fp64) {
+  return p->nx < (fp64 ? 64 : 96) && p->nang <= 256 &&
+         (long long)p->nang * p->nx * p->nx <= (fp64 ? 1 << 16 : 1 << 18);
+}
+
 // grid = E^T of all slices.  The work counter of the launch is a voxel of the
 // output that no tap reaches, (x, y, z) = (NX, 0, 0): the plan may run on
 // several streams at once, so the counter has to be the call's own.
 template <class F>
 int fs_adjoint(const spi_fslice_plan* p, const void* slices, void* grid, size_t voxel, cudaStream_t s) {
   SPI_CUDA(cudaMemsetAsync(grid, 0, fs_grid_elems(p) * voxel, s));
+  if (fs_small(p, F::D)) {
+    const long long rows = ((long long)p->nang * p->n + 7) / 8;
+    fs_taps_kernel<F::D><<<(int)std::min<long long>(rows, fs_blocks(p)), 256, kFsSmem, s>>>(
+        static_cast<const float2*>(slices), grid, p->sl, p->nang, p->nx, p->tab, p->fltb);
+    SPI_TRY(check_kernel("fs_taps_kernel"));
+    p->ctx->count();
+    return 0;
+  }
   auto* work = reinterpret_cast<unsigned long long*>(static_cast<char*>(grid) + (size_t)p->nx * voxel);
   SPI_TRY(fs_insert<F>(p, slices, grid, 0, p->nang, work, s));
   SPI_CUDA(cudaMemsetAsync(work, 0, sizeof(*work), s));

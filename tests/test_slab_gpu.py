@@ -107,9 +107,11 @@ def test_columns_not_finite(ctx):
     assert synth.rel_l2(w, wd) <= 1e-6
 
 
-@pytest.mark.parametrize("nx,nang", [(8, 3), (15, 20), (16, 1), (17, 20), (40, 300)])
+# few slices go tap by tap, more by columns: from 257 on, FP64 from 41 on at 40^3
+@pytest.mark.parametrize("nx,nang", [(8, 3), (15, 20), (16, 1), (17, 20), (40, 300), (40, 41), (8, 300), (15, 300),
+                                     (16, 300), (17, 300), (16, 256), (16, 257), (64, 2), (96, 2)])
 def test_fourier_slice_pair(ctx, orc, nx, nang):
-    """E and E^T by tiles and columns at the edges of both, FP32 within 2e-6 (as
+    """E and E^T at the edges of their tiles and of the routes, FP32 within 2e-6 (as
     above; E sums 64 products) and FP64 within 1e-12 of the oracle pair."""
     import torch
 
@@ -201,20 +203,21 @@ def test_fourier_slice_normal_without_room(ctx):
         plan.close()
 
 
+@pytest.mark.parametrize("count", [12, 300])
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
-def test_fourier_slice_angles_not_finite(ctx, bad):
+def test_fourier_slice_angles_not_finite(ctx, bad, count):
     """A slice with an angle that is not finite has no taps: E writes zeros, E^T and
     the normal operators leave it out, the other slices are as without it."""
     import torch
 
     from spider_b200 import autograd
     nx = 24
-    good = _angles(12, 6)
+    good = _angles(count, 6)
     ang = np.repeat(good, 2, axis=0)
-    for i in range(12):
+    for i in range(count):
         ang[2 * i + 1, i % 3] = bad
     X = torch.randn((2 * nx, 2 * nx, nx + 1, 2), device="cuda")
-    T = torch.randn((24, 2 * nx, nx + 1, 2), device="cuda")
+    T = torch.randn((2 * count, 2 * nx, nx + 1, 2), device="cuda")
     plan, ref = autograd.FourierSlicePlan(nx, ang, ctx=ctx), autograd.FourierSlicePlan(nx, good, ctx=ctx)
     try:
         for fwd, x in (("forward", X), ("forward64", X.double())):
